@@ -102,7 +102,11 @@ struct SceneView {
     const int32_t* __restrict__ tri_id;
     const GNode8* __restrict__ nodes8;  // the 8-wide tree of the same leaves, or null
     const int32_t* __restrict__ tie;    // per slot: rank in the reference's walk order, or null
+    const unsigned long long* __restrict__ horizon;  // per slot: a byte per octant of directions (horizon.cu)
 };
+
+// Horizon bytes are multiples of 1 / kHorizonUnit of d.n; 255 is out of any ray's reach.
+constexpr float kHorizonUnit = 254.0f;
 
 // --------------------------------------------------------------- plan data
 // One (job, angle) of a plan.  Frames are computed on the host in FP64.

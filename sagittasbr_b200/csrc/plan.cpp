@@ -459,6 +459,15 @@ sbr_status plan_create(sbr_scene* const* scenes, size_t n_scenes, const int32_t*
     p->n_rays_clipped = tot.n_rays_clipped;
     p->n_rays_grid = tot.n_rays_grid;
     p->n_pol = p->pol == SBR_POL_HHVV ? 2 : 1;
+    // a refitted scene has no horizons: a plan that launches enough rays to pay for them
+    // (5 to 20 ns a triangle against 50 to 100 ps a ray, measured on B200) brings them back
+    if (!p->multi && p->prec != SBR_PREC_FP32 && p->n_rays_clipped >= 200 * s->ntris) {
+        sbr_status st = build_horizons(s);
+        if (st != SBR_OK) {
+            release(p);
+            return st;
+        }
+    }
     if (p->n_pol == 2) {
         // per angle: HH / VV unit vectors and the reference launch plane; the
         // accumulator units are per (sample, polarisation)

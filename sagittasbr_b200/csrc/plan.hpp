@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "common.hpp"
@@ -29,6 +30,9 @@ struct sbr_scene {
     sbr::GTri64* d_tris64 = nullptr;
     int32_t* d_tri_id = nullptr;
     int32_t* d_tie = nullptr;        // exact-tie ranks (coincident faces of opposite winding), or null
+    unsigned long long* d_horizon = nullptr;  // per slot: escape elevations by octant (horizon.cu)
+    bool horizon_built = false;      // false after a refit: all bytes 255, every ray walks
+    std::mutex horizon_mu;
     float* d_xyz = nullptr;          // caller vertices and triangles, uploaded for the adjoint
     uint32_t* d_idx = nullptr;
     uint32_t* d_err = nullptr;
@@ -46,7 +50,7 @@ struct sbr_scene {
     float* d_tri_box = nullptr;
     int64_t device_bytes = 0;
 
-    sbr::SceneView view() const { return sbr::SceneView{d_nodes, d_tris, d_tris64, d_tri_id, d_nodes8, d_tie}; }
+    sbr::SceneView view() const { return sbr::SceneView{d_nodes, d_tris, d_tris64, d_tri_id, d_nodes8, d_tie, d_horizon}; }
 };
 
 struct sbr_plan {
@@ -147,4 +151,8 @@ sbr_status trace_list_launch(sbr_plan* pl, const int32_t* d_rays, long long n, s
 int max_freqs_per_job();
 sbr_status ensure_fp64(sbr_scene* s);
 sbr_status ensure_adjoint_data(sbr_scene* s);
+// Computes the scene's horizons unless it holds them, and waits for them.
+sbr_status build_horizons(sbr_scene* s);
+// Takes them back, in stream order, so that every ray walks (plans that exist see it).
+sbr_status clear_horizons(sbr_scene* s);
 }  // namespace sbr

@@ -16,13 +16,14 @@ struct RayF {
     double L;       // FP64 path (mixed)
     float dist32;   // FP32 path (reference FP32 arithmetic)
     int count;
-    int zidx;       // entry of this ray in the first-hit buffer
+    int zidx;       // entry of this ray in the first-hit buffer; -1: known to leave the scene
 };
 struct RayD {
     D3 o, d, nl, dl;
     double cosl;
     double L;
     int count;
+    bool gone;      // known to leave the scene
 };
 
 // What the PO epilogue needs from a finished ray.
@@ -94,6 +95,16 @@ __device__ __forceinline__ F3 primary_origin(const Segment& G, const JobConst& J
     }
 }
 
+// Whether a ray that triangle `slot` reflected (n: its normal, d: the new direction,
+// unit) is known to meet nothing: it left the front side (cosl > 0) and rises above
+// the triangle's horizon in its octant of directions (horizon.cu).  Its next query
+// then returns a miss without a walk.
+__device__ __forceinline__ bool leaves_scene(const SceneView& S, int slot, float cosl, float dx, float dy, float dz,
+                                             float dn) {
+    const unsigned o = (__float_as_uint(dx) >> 31) | (__float_as_uint(dy) >> 31) << 1 | (__float_as_uint(dz) >> 31) << 2;
+    return cosl > 0.0f && dn * kHorizonUnit > float(unsigned(__ldg(S.horizon + slot) >> (8 * o)) & 255u);
+}
+
 // First-hit buffer entry of ray (i, j): tile-major, the lane of the 4x8 block last.
 __device__ __forceinline__ int zindex(const Segment& G, int i, int j) {
     const int bi = i - G.i0, bj = j - G.j0;
@@ -104,7 +115,7 @@ template <int PREC>
 __device__ __forceinline__ void start_f(RayF& r, const Segment& G, const JobConst& J, int i, int j) {
     r.o = primary_origin<PREC>(G, J, i, j);
     r.L = PREC == SBR_PREC_FP32 ? 0.0 : G.shift;
-    r.zidx = zindex(G, i, j);
+    r.zidx = zindex(G, i, j) & 0x7fffffff;  // (walking plans do not use it; it may have wrapped there)
     r.d = f3(G.rdf[0], G.rdf[1], G.rdf[2]);
     r.nl = f3(0, 0, 0);
     r.dl = f3(0, 0, 0);
@@ -125,6 +136,7 @@ constexpr unsigned long long kZWalk = 0xfffffffe00000000ull;
 template <int PREC, bool REC, bool POL, bool W8 = false, bool SPEC = false>
 __device__ __forceinline__ bool step_f(RayF& r, PolF& e, const SceneView& S, int maxB, uint32_t& err,
                                        sbr_ray_record* rec, unsigned long long* zbuf, unsigned mask = 0u) {
+    if (PREC == SBR_PREC_MIXED && r.zidx < 0) return true;
     float tB = 1e20f;
     int slot;
     const unsigned long long key = (zbuf != nullptr && r.count == 0) ? zbuf[r.zidx] : kZWalk;
@@ -160,6 +172,8 @@ __device__ __forceinline__ bool step_f(RayF& r, PolF& e, const SceneView& S, int
     const F3 p = fma3(tB, r.d, r.o);
     r.d = reflect_dir(r.d, n);
     r.o = nudge(p, n);
+    if (PREC == SBR_PREC_MIXED && r.count < maxB && leaves_scene(S, slot, r.cosl, r.d.x, r.d.y, r.d.z, dot(r.d, n)))
+        r.zidx = -1;
     return r.count >= maxB;
 }
 
@@ -192,11 +206,13 @@ __device__ __forceinline__ void start_d(RayD& r, const Segment& G, const JobCons
     r.cosl = 0.0;
     r.L = G.shift;
     r.count = 0;
+    r.gone = false;
 }
 
 template <bool REC, bool POL>
 __device__ __forceinline__ bool step_d(RayD& r, PolD& e, const SceneView& S, int maxB, uint32_t& err,
                                        sbr_ray_record* rec) {
+    if (r.gone) return true;
     double tB = 1e20;
     const int slot = Walker<true>::closest(S, r.o, r.d, 1.0e-3, tB, err);
     if (slot < 0) return true;
@@ -219,6 +235,7 @@ __device__ __forceinline__ bool step_d(RayD& r, PolD& e, const SceneView& S, int
     const D3 p = r.o + tB * r.d;
     r.d = reflect_dir(r.d, n);
     r.o = nudge(p, n);
+    r.gone = r.count < maxB && leaves_scene(S, slot, float(r.cosl), float(r.d.x), float(r.d.y), float(r.d.z), float(dot(r.d, n)));
     return r.count >= maxB;
 }
 

@@ -152,6 +152,7 @@ extern "C" sbr_status sbr_scene_update_vertices(sbr_scene* s, const float* xyz, 
         s->device_bytes += (int64_t)(nb + bb);
     }
     s->xyz.assign(xyz, xyz + 3 * nverts);
+    if ((st = clear_horizons(s)) != SBR_OK) return st;
     cudaStream_t st_ = s->stream;
     SBR_CUDA(cudaMemcpyAsync(s->d_xyz, s->xyz.data(), s->xyz.size() * sizeof(float), cudaMemcpyHostToDevice, st_));
     const unsigned gt = (unsigned)((s->ntris + kRefitThreads - 1) / kRefitThreads);

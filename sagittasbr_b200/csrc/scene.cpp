@@ -70,6 +70,7 @@ void free_scene(sbr_scene* s) {
     cudaFree(s->d_tris64);
     cudaFree(s->d_tri_id);
     cudaFree(s->d_tie);
+    cudaFree(s->d_horizon);
     cudaFree(s->d_xyz);
     cudaFree(s->d_idx);
     cudaFree(s->d_refit_nodes);
@@ -432,6 +433,14 @@ sbr_status sbr_scene_create(const float* xyz, size_t nverts, const uint32_t* tri
         if ((e = cudaMemcpy(s->d_nodes8, g8.data(), nb8, cudaMemcpyHostToDevice)) != cudaSuccess)
             return bail(cuda_fail(e, "8-wide node upload"));
         s->device_bytes += (int64_t)nb8;
+    }
+    {
+        const size_t hb = sizeof(unsigned long long) * ntris;
+        if ((e = cudaMalloc(&s->d_horizon, hb)) != cudaSuccess)
+            return bail(fail(SBR_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(e)));
+        sbr_status st = build_horizons(s);
+        if (st != SBR_OK) return bail(st);
+        s->device_bytes += (int64_t)hb;
     }
     if (o.want_fp64 > 0) {
         sbr_status st = ensure_fp64(s);
