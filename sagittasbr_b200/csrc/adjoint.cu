@@ -243,15 +243,15 @@ const void* pick_adjoint(int prec) {
     }
 }
 
-// Device buffers of one adjoint call, released on every exit path.
+// Device block of one adjoint call, given back on every exit path.
 struct AdjointBuffers {
-    double* cot = nullptr;
-    double* grad_pos = nullptr;
-    double* grad_k = nullptr;
+    int device;
+    cudaStream_t stream;
+    char* block = nullptr;
     ~AdjointBuffers() {
-        cudaFree(cot);
-        cudaFree(grad_pos);
-        cudaFree(grad_k);
+        if (!block) return;
+        if (cudaStreamSynchronize(stream) != cudaSuccess) cudaDeviceSynchronize();
+        pool_free(device, block);
     }
 };
 
@@ -263,8 +263,8 @@ sbr_status ensure_adjoint_data(sbr_scene* s) {
     sbr::DeviceGuard device_guard;
     SBR_CUDA(cudaSetDevice(s->device));
     const size_t vb = s->xyz.size() * sizeof(float), ib = s->idx.size() * sizeof(uint32_t);
-    if (cudaMalloc(&s->d_xyz, vb) != cudaSuccess || cudaMalloc(&s->d_idx, ib) != cudaSuccess)
-        return fail(SBR_ERR_OOM, "cudaMalloc of the adjoint mesh copy failed");
+    if (pool_alloc(s->device, &s->d_xyz, vb) != cudaSuccess || pool_alloc(s->device, &s->d_idx, ib) != cudaSuccess)
+        return fail(SBR_ERR_OOM, "allocation of the adjoint mesh copy failed");
     SBR_CUDA(cudaMemcpy(s->d_xyz, s->xyz.data(), vb, cudaMemcpyHostToDevice));
     SBR_CUDA(cudaMemcpy(s->d_idx, s->idx.data(), ib, cudaMemcpyHostToDevice));
     s->device_bytes += (int64_t)(vb + ib);
@@ -298,15 +298,17 @@ extern "C" sbr_status sbr_adjoint(sbr_scene* s, const sbr_job* jobs, size_t n_jo
     if ((st = ensure_adjoint_data(s)) != SBR_OK) return st;
 
     const size_t nv3 = s->xyz.size(), ns = (size_t)p->n_samples;
-    AdjointBuffers B;
     cudaStream_t stream = p->stream;
-    if (cudaMalloc(&B.cot, std::max<size_t>(1, 2 * ns) * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&B.grad_pos, nv3 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&B.grad_k, std::max<size_t>(1, ns) * sizeof(double)) != cudaSuccess)
-        return fail(SBR_ERR_OOM, "adjoint buffers");
-    if (ns) SBR_CUDA(cudaMemcpyAsync(B.cot, cot, 2 * ns * sizeof(double), cudaMemcpyHostToDevice, stream));
-    SBR_CUDA(cudaMemsetAsync(B.grad_pos, 0, nv3 * sizeof(double), stream));
-    SBR_CUDA(cudaMemsetAsync(B.grad_k, 0, std::max<size_t>(1, ns) * sizeof(double), stream));
+    AdjointBuffers B{s->device, stream};
+    Parts parts;
+    const size_t pos_at = parts.add(nv3 * sizeof(double)), k_at = parts.add(ns * sizeof(double)), zero_b = parts.add(0),
+                 cot_at = parts.add(2 * ns * sizeof(double));
+    if (pool_alloc(s->device, &B.block, parts.size()) != cudaSuccess) return fail(SBR_ERR_OOM, "adjoint buffers");
+    double* const d_pos = reinterpret_cast<double*>(B.block + pos_at);
+    double* const d_k = reinterpret_cast<double*>(B.block + k_at);
+    double* const d_cot = reinterpret_cast<double*>(B.block + cot_at);
+    if (ns) SBR_CUDA(cudaMemcpyAsync(d_cot, cot, 2 * ns * sizeof(double), cudaMemcpyHostToDevice, stream));
+    SBR_CUDA(cudaMemsetAsync(B.block, 0, zero_b, stream));
 
     if (p->n_items > 0) {
         const void* fn = pick_adjoint(p->prec);
@@ -325,17 +327,17 @@ extern "C" sbr_status sbr_adjoint(sbr_scene* s, const sbr_job* jobs, size_t n_jo
         a.freqs = p->d_freqs;
         a.n_items = p->n_items;
         a.queue = p->d_queue;
-        a.cot = B.cot;
-        a.grad_pos = B.grad_pos;
-        a.grad_k = B.grad_k;
+        a.cot = d_cot;
+        a.grad_pos = d_pos;
+        a.grad_k = d_k;
         a.err = s->d_err;
         a.cancel = s->d_cancel;
         void* args[] = {&a};
         SBR_CUDA(cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(kCtaThreads), args, 0, stream));
     }
     std::vector<double> gp(nv3), gk(ns);
-    SBR_CUDA(cudaMemcpyAsync(gp.data(), B.grad_pos, nv3 * sizeof(double), cudaMemcpyDeviceToHost, stream));
-    if (ns) SBR_CUDA(cudaMemcpyAsync(gk.data(), B.grad_k, ns * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    SBR_CUDA(cudaMemcpyAsync(gp.data(), d_pos, nv3 * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    if (ns) SBR_CUDA(cudaMemcpyAsync(gk.data(), d_k, ns * sizeof(double), cudaMemcpyDeviceToHost, stream));
     SBR_CUDA(cudaStreamSynchronize(stream));
     uint32_t e = 0;
     SBR_CUDA(cudaMemcpy(&e, s->d_err, sizeof(e), cudaMemcpyDeviceToHost));

@@ -397,14 +397,17 @@ extern "C" sbr_status sbr_error_bound(sbr_scene* s, const sbr_job* jobs, size_t 
     unsigned long long* d_queue = nullptr;
     std::vector<double> acc(8 * (size_t)std::max<int64_t>(p->n_segs, 1), 0.0);
     std::vector<double> dfield(2 * (size_t)std::max<int64_t>(p->n_samples, 1), 0.0);
-    cudaError_t e = cudaMalloc(&d_acc, acc.size() * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&d_dfield, dfield.size() * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&d_queue, sizeof(unsigned long long));
+    Parts parts;
+    const size_t acc_at = parts.add(acc.size() * sizeof(double)), df_at = parts.add(dfield.size() * sizeof(double)),
+                 queue_at = parts.add(sizeof(unsigned long long));
+    char* block = nullptr;
+    cudaError_t e = pool_alloc(p->device, &block, parts.size());
     if (e != cudaSuccess) st = fail(SBR_ERR_OOM, "error-bound accumulators");
     if (st == SBR_OK) {
-        e = cudaMemsetAsync(d_acc, 0, acc.size() * sizeof(double), p->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(d_dfield, 0, dfield.size() * sizeof(double), p->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(d_queue, 0, sizeof(unsigned long long), p->stream);
+        d_acc = reinterpret_cast<double*>(block + acc_at);
+        d_dfield = reinterpret_cast<double*>(block + df_at);
+        d_queue = reinterpret_cast<unsigned long long*>(block + queue_at);
+        e = cudaMemsetAsync(block, 0, parts.size(), p->stream);
         if (e != cudaSuccess) st = cuda_fail(e, "error-bound clear");
     }
     if (st == SBR_OK && p->n_items > 0) {
@@ -477,9 +480,8 @@ extern "C" sbr_status sbr_error_bound(sbr_scene* s, const sbr_job* jobs, size_t 
             }
         }
     }
-    cudaFree(d_acc);
-    cudaFree(d_dfield);
-    cudaFree(d_queue);
+    if (cudaStreamSynchronize(p->stream) != cudaSuccess) cudaDeviceSynchronize();
+    pool_free(p->device, block);
     sbr_plan_destroy(p);
     return st;
 }

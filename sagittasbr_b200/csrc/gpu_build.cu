@@ -25,6 +25,7 @@
 
 #include "bvh_build.hpp"
 #include "common.hpp"
+#include "devpool.hpp"
 
 namespace sbr {
 namespace {
@@ -447,11 +448,6 @@ __global__ void k_assign(Work W, Level L) {
     W.node_of[p] = c < 0 ? -1 : (p < L.s[j] + L.left_count[j] ? c : c + 1);
 }
 
-template <typename T>
-cudaError_t dalloc(T** p, size_t count) {
-    return cudaMalloc(reinterpret_cast<void**>(p), sizeof(T) * std::max<size_t>(count, 1));
-}
-
 }  // namespace
 
 // See bvh_build.hpp.  Returns false (with the CUDA error in *err) if a CUDA call fails.
@@ -468,21 +464,16 @@ bool build_sah_gpu(const std::vector<float>& tri_lo, const std::vector<float>& t
 
     Work W{};
     Level L[2]{};
-    std::vector<void*> owned;
-    cudaError_t e = cudaSuccess;
+    // all work arrays in one block: their sizes first, then their addresses
+    Parts parts;
+    std::vector<std::pair<void**, size_t>> owned;
     auto A = [&](auto** p, size_t count) {
-        if (e == cudaSuccess) {
-            e = dalloc(p, count);
-            if (e == cudaSuccess) owned.push_back(*p);
-        }
+        owned.emplace_back(reinterpret_cast<void**>(p), parts.add(sizeof(**p) * count));
     };
     float *lo, *hi, *ce;
     A(&lo, 3 * (size_t)n);
     A(&hi, 3 * (size_t)n);
     A(&ce, 3 * (size_t)n);
-    W.lo = lo;
-    W.hi = hi;
-    W.cen = ce;
     A(&W.idx, n);
     A(&W.tmp, n);
     A(&W.node_of, n);
@@ -509,12 +500,25 @@ bool build_sah_gpu(const std::vector<float>& tri_lo, const std::vector<float>& t
         A(&l.left_count, cap);
         A(&l.child_slot, cap);
     }
+    int device = 0;
+    char* block = nullptr;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = pool_alloc(device, &block, parts.size());
+    if (e != cudaSuccess) {
+        *err = e;
+        return false;
+    }
+    for (auto& o : owned) *o.first = block + o.second;
+    W.lo = lo;
+    W.hi = hi;
+    W.cen = ce;
     W.n = n;
     W.bins = B;
     W.leaf_size = opt.leaf_size;
     W.max_leaf = opt.max_leaf;
     auto cleanup = [&]() {
-        for (void* p : owned) cudaFree(p);
+        if (cudaStreamSynchronize(stream) != cudaSuccess) cudaDeviceSynchronize();
+        pool_free(device, block);
     };
     if (e == cudaSuccess) e = cudaMemcpyAsync(lo, tri_lo.data(), 12 * (size_t)n, cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(hi, tri_hi.data(), 12 * (size_t)n, cudaMemcpyHostToDevice, stream);

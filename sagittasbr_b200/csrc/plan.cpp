@@ -57,68 +57,32 @@ Fr<R> frame(double thetaDeg, double phiDeg, R G) {
     return f;
 }
 
-template <class T>
-sbr_status upload(T** d, const std::vector<T>& h, int64_t& bytes) {
-    size_t n = std::max<size_t>(h.size(), 1) * sizeof(T);
-    cudaError_t e = cudaMalloc(d, n);
-    if (e != cudaSuccess) return fail(SBR_ERR_OOM, "plan allocation failed");
-    bytes += (int64_t)n;
-    if (!h.empty()) SBR_CUDA(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
-    return SBR_OK;
-}
-
-template <class T>
-sbr_status dalloc(T** d, size_t count, int64_t& bytes) {
-    size_t n = std::max<size_t>(count, 1) * sizeof(T);
-    cudaError_t e = cudaMalloc(d, n);
-    if (e != cudaSuccess) return fail(SBR_ERR_OOM, "plan allocation failed");
-    bytes += (int64_t)n;
-    return SBR_OK;
-}
-// Zeroed on the plan's stream, so the plan's first launches come after the zeros
-// (a cudaMemset on the legacy stream is not ordered with a non-blocking stream).
-template <class T>
-sbr_status zalloc(T** d, size_t count, int64_t& bytes, cudaStream_t st) {
-    sbr_status r = dalloc(d, count, bytes);
-    if (r != SBR_OK) return r;
-    SBR_CUDA(cudaMemsetAsync(*d, 0, std::max<size_t>(count, 1) * sizeof(T), st));
-    return SBR_OK;
-}
-
 void release(sbr_plan* p) {
     if (!p) return;
     sbr::DeviceGuard device_guard;
-    cudaSetDevice(p->scene->device);
-    if (p->stream) cudaStreamSynchronize(p->stream);
+    cudaSetDevice(p->device);
+    // the blocks go back to the pool: nothing may use them any more
+    if (p->handed_out || (p->stream && cudaStreamSynchronize(p->stream) != cudaSuccess)) cudaDeviceSynchronize();
     if (p->graph) cudaGraphExecDestroy(p->graph);
-    cudaFree(p->d_segs);
-    cudaFree(p->d_seg_base);
-    cudaFree(p->d_jobs);
-    cudaFree(p->d_freqs);
-    cudaFree(p->d_quantum);
-    cudaFree(p->d_acc);
-    cudaFree(p->d_acc_stats);
-    cudaFree(p->d_field);
-    cudaFree(p->d_stats);
-    cudaFree(p->d_queue);
-    cudaFree(p->d_zbuf);
-    cudaFree(p->d_tile_cnt);
-    cudaFree(p->d_tile_list);
-    cudaFree(p->d_segpol);
-    cudaFree(p->d_scenes);
+    pool_free(p->device, p->block);
+    pool_free(p->device, p->raster_block);
     if (p->ev0) cudaEventDestroy(p->ev0);
     if (p->ev1) cudaEventDestroy(p->ev1);
     delete p;
 }
 
-sbr_status check_device_errors(sbr_plan* p) {
-    uint32_t e = 0;
-    SBR_CUDA(cudaMemcpy(&e, p->d_err, sizeof(e), cudaMemcpyDeviceToHost));
+// Status of an error word read back, which is cleared when it held one.
+sbr_status report_device_errors(sbr_plan* p, uint32_t e) {
     if (e) clear_device_word(p->d_err);
     if (e & DEV_ERR_CANCEL) return fail(SBR_ERR_CANCELLED, "run cancelled");
     if (e & DEV_ERR_BUDGET) return fail(SBR_ERR_TIMEOUT, "traversal iteration budget exceeded");
     if (e & DEV_ERR_STACK) return fail(SBR_ERR_STACK, "traversal stack overflow");
     return SBR_OK;
+}
+sbr_status check_device_errors(sbr_plan* p) {
+    uint32_t e = 0;
+    SBR_CUDA(cudaMemcpy(&e, p->d_err, sizeof(e), cudaMemcpyDeviceToHost));
+    return report_device_errors(p, e);
 }
 
 }  // namespace
@@ -427,6 +391,7 @@ sbr_status plan_create(sbr_scene* const* scenes, size_t n_scenes, const int32_t*
 
     sbr_plan* p = new sbr_plan();
     p->scene = s;
+    p->device = s->device;
     p->blocks_per_item = o.blocks_per_item;
     p->multi = job_scene != nullptr;
     if (p->multi)
@@ -441,7 +406,6 @@ sbr_status plan_create(sbr_scene* const* scenes, size_t n_scenes, const int32_t*
     p->scene_view = s->view();
     p->node_width = !job_scene && ((o.node_width == 0 && s->d_nodes8) || o.node_width == 8) ? 8 : 4;
     if (p->node_width == 4) p->scene_view.nodes8 = nullptr;  // the sweep kernel walks the 4-wide tree
-    p->d_err = s->d_err;
     p->d_cancel = s->d_cancel;
 
     PlanSink sink(p);
@@ -498,15 +462,20 @@ sbr_status plan_create(sbr_scene* const* scenes, size_t n_scenes, const int32_t*
     p->raster = o.mode == SBR_MODE_BATCHED && o.precision == SBR_PREC_MIXED && p->n_items > 0 && !p->multi &&
                 (o.first_hit == SBR_FIRST_HIT_RASTER || (o.first_hit == SBR_FIRST_HIT_AUTO && dense));
     if (p->raster) {
-        // per tile: 32 first-hit entries (8 B), a count and `cap` list entries (4 B);
-        // a chunk holds at most 8 GiB of them (or one segment)
+        // per tile: 32 first-hit entries (8 B), a count and `cap` list entries (4 B).  A
+        // chunk holds 1 GiB of them, which the memory pool keeps from one call to the next
+        // (a 181-azimuth narrow sweep's 2.8 GB in one piece cost 2.6 ms of mapping a call),
+        // and more, up to 8 GiB, until it has 12 segments: every chunk ends with a wait for
+        // its slowest warps (0.5 ms an azimuth when 10 azimuths of the 12,222^2 grid,
+        // 0.55 GB each, went one by one instead of together: 44.7 against 31.9 ms).
         p->tile_cap = o.tile_cap > 0 ? (uint32_t)o.tile_cap : 48u;
-        const int64_t budget = (int64_t(8) << 30) / (32 * 8 + 4 + 4 * (int64_t)p->tile_cap);
+        const int64_t tile_bytes = 32 * 8 + 4 + 4 * (int64_t)p->tile_cap;
+        const int64_t budget = (int64_t(1023) << 20) / tile_bytes, most = (int64_t(8) << 30) / tile_bytes;
         sbr_plan::Chunk c{0, 0, 0, 0, 0, 0};
         for (size_t g = 0; g < p->segs.size(); ++g) {
-            const int64_t tiles = p->segs[g].blocks;
+            const int64_t tiles = p->segs[g].blocks, held = c.seg_end - c.seg_begin;
             // (the binning launch's grid.y is the chunk's segment count: at most 65535)
-            if (c.seg_end > c.seg_begin && (c.tiles + tiles > budget || c.seg_end - c.seg_begin >= 65535)) {
+            if (held > 0 && (c.tiles + tiles > most || (c.tiles + tiles > budget && held >= 12) || held >= 65535)) {
                 c.item_end = p->seg_base[c.seg_end];
                 p->chunks.push_back(c);
                 c = sbr_plan::Chunk{c.seg_end, c.seg_end, p->seg_base[c.seg_end], 0, 0, 0};
@@ -525,47 +494,85 @@ sbr_status plan_create(sbr_scene* const* scenes, size_t n_scenes, const int32_t*
         }
     }
 
-    sbr_status st;
-    int64_t& b = p->device_bytes;
     if (p->raster) {
         // every entry of a chunk is written by its tile raster before the trace reads it
-        const int64_t b0 = b;
-        if ((st = dalloc(&p->d_zbuf, (size_t)p->zbuf_elems, b)) != SBR_OK ||
-            (st = dalloc(&p->d_tile_cnt, (size_t)p->tiles_max, b)) != SBR_OK ||
-            (st = dalloc(&p->d_tile_list, (size_t)p->tiles_max * p->tile_cap, b)) != SBR_OK) {
-            if (o.first_hit == SBR_FIRST_HIT_RASTER) {
-                release(p);
-                return st;
-            }
+        Parts parts;
+        const size_t zb = parts.add((size_t)p->zbuf_elems * sizeof(unsigned long long)),
+                     cn = parts.add((size_t)p->tiles_max * sizeof(uint32_t)),
+                     ls = parts.add((size_t)p->tiles_max * p->tile_cap * sizeof(int32_t));
+        char* r = nullptr;
+        if (pool_alloc(p->device, &r, parts.size()) == cudaSuccess) {
+            p->raster_block = r;
+            p->d_zbuf = reinterpret_cast<unsigned long long*>(r + zb);
+            p->d_tile_cnt = reinterpret_cast<uint32_t*>(r + cn);
+            p->d_tile_list = reinterpret_cast<int32_t*>(r + ls);
+            p->device_bytes += (int64_t)parts.size();
+        } else if (o.first_hit == SBR_FIRST_HIT_RASTER) {
+            release(p);
+            return fail(SBR_ERR_OOM, "plan allocation failed");
+        } else {
             // chosen automatically: without room for its buffers the plan walks instead
-            // (a failed cudaMalloc is not sticky; its error is cleared here)
-            cudaGetLastError();
-            cudaFree(p->d_zbuf);
-            cudaFree(p->d_tile_cnt);
-            cudaFree(p->d_tile_list);
-            p->d_zbuf = nullptr;
-            p->d_tile_cnt = nullptr;
-            p->d_tile_list = nullptr;
-            b = b0;
             p->raster = false;
             p->chunks.clear();
             p->zbuf_elems = 0;
             p->tiles_max = 0;
-            st = SBR_OK;
         }
     }
-    if ((st = upload(&p->d_segs, p->segs, b)) != SBR_OK || (st = upload(&p->d_seg_base, p->seg_base, b)) != SBR_OK ||
-        (st = upload(&p->d_jobs, p->jobs, b)) != SBR_OK || (st = upload(&p->d_freqs, p->freqs, b)) != SBR_OK ||
-        (st = upload(&p->d_quantum, p->quantum, b)) != SBR_OK ||
-        (p->n_pol == 2 && (st = upload(&p->d_segpol, p->segpol, b)) != SBR_OK) ||
-        (p->multi && (st = upload(&p->d_scenes, p->scene_views, b)) != SBR_OK) ||
-        (st = zalloc(&p->d_acc, 2 * (size_t)p->n_samples * p->n_pol * kAccReplicas, b, p->stream)) != SBR_OK ||
-        (st = zalloc(&p->d_acc_stats, 4 * (size_t)p->n_segs, b, p->stream)) != SBR_OK ||
-        (st = zalloc(&p->d_field, 2 * (size_t)p->n_samples * p->n_pol, b, p->stream)) != SBR_OK ||
-        (st = zalloc(&p->d_stats, 4 * (size_t)p->n_segs, b, p->stream)) != SBR_OK ||
-        (st = zalloc(&p->d_queue, 1 + (size_t)p->n_samples + p->chunks.size(), b, p->stream)) != SBR_OK) {
+    // one block: the tables (copied up in one piece), then what starts out zero -- on the
+    // plan's stream, so that its launches come after both -- with the error word, fields
+    // and counters last, next to one another (copied down in one piece)
+    Parts parts;
+    const size_t seg_b = p->segs.size() * sizeof(Segment), base_b = p->seg_base.size() * sizeof(int64_t),
+                 job_b = p->jobs.size() * sizeof(JobConst), freq_b = p->freqs.size() * sizeof(FreqConst),
+                 quant_b = p->quantum.size() * sizeof(double), pol_b = p->segpol.size() * sizeof(SegPol),
+                 view_b = p->scene_views.size() * sizeof(SceneView);
+    const size_t seg_at = parts.add(seg_b), base_at = parts.add(base_b), job_at = parts.add(job_b),
+                 freq_at = parts.add(freq_b), quant_at = parts.add(quant_b), pol_at = parts.add(pol_b),
+                 view_at = parts.add(view_b), tables = parts.add(0);
+    const size_t n_out = (size_t)p->n_samples * p->n_pol;
+    const size_t acc_at = parts.add(2 * n_out * kAccReplicas * sizeof(unsigned long long)),
+                 acc_stats_at = parts.add(4 * (size_t)p->n_segs * sizeof(unsigned long long)),
+                 queue_at = parts.add((1 + (size_t)p->n_samples + p->chunks.size()) * sizeof(unsigned long long)),
+                 err_at = parts.add(sizeof(uint32_t)), field_at = parts.add(2 * n_out * sizeof(double)),
+                 stats_at = parts.add(4 * (size_t)p->n_segs * sizeof(unsigned long long));
+    char* b = nullptr;
+    if (pool_alloc(p->device, &b, parts.size()) != cudaSuccess) {
         release(p);
-        return st;
+        return fail(SBR_ERR_OOM, "plan allocation failed");
+    }
+    p->block = b;
+    p->device_bytes += (int64_t)parts.size();
+    p->d_segs = reinterpret_cast<Segment*>(b + seg_at);
+    p->d_seg_base = reinterpret_cast<int64_t*>(b + base_at);
+    p->d_jobs = reinterpret_cast<JobConst*>(b + job_at);
+    p->d_freqs = reinterpret_cast<FreqConst*>(b + freq_at);
+    p->d_quantum = reinterpret_cast<double*>(b + quant_at);
+    if (p->n_pol == 2) p->d_segpol = reinterpret_cast<SegPol*>(b + pol_at);
+    if (p->multi) p->d_scenes = reinterpret_cast<SceneView*>(b + view_at);
+    p->d_acc = reinterpret_cast<unsigned long long*>(b + acc_at);
+    p->d_acc_stats = reinterpret_cast<unsigned long long*>(b + acc_stats_at);
+    p->d_queue = reinterpret_cast<unsigned long long*>(b + queue_at);
+    p->d_err = reinterpret_cast<uint32_t*>(b + err_at);
+    p->d_field = reinterpret_cast<double*>(b + field_at);
+    p->d_stats = reinterpret_cast<unsigned long long*>(b + stats_at);
+    p->results_bytes = parts.size() - err_at;
+    p->stats_at = stats_at - err_at;
+    std::vector<char> up(tables);
+    auto put = [&](size_t at, const void* src, size_t n) {
+        if (n) std::memcpy(up.data() + at, src, n);
+    };
+    put(seg_at, p->segs.data(), seg_b);
+    put(base_at, p->seg_base.data(), base_b);
+    put(job_at, p->jobs.data(), job_b);
+    put(freq_at, p->freqs.data(), freq_b);
+    put(quant_at, p->quantum.data(), quant_b);
+    put(pol_at, p->segpol.data(), pol_b);
+    put(view_at, p->scene_views.data(), view_b);
+    cudaError_t ue = tables ? cudaMemcpyAsync(b, up.data(), tables, cudaMemcpyHostToDevice, p->stream) : cudaSuccess;
+    if (ue == cudaSuccess) ue = cudaMemsetAsync(b + tables, 0, parts.size() - tables, p->stream);
+    if (ue != cudaSuccess) {
+        release(p);
+        return cuda_fail(ue, "plan tables");
     }
     cudaError_t e;
     if ((e = cudaEventCreate(&p->ev0)) != cudaSuccess || (e = cudaEventCreate(&p->ev1)) != cudaSuccess) {
@@ -594,7 +601,7 @@ sbr_status sbr_plan_create_multi(sbr_scene* const* scenes, size_t n_scenes, cons
 sbr_status sbr_plan_execute(sbr_plan* p) {
     if (!p) return fail(SBR_ERR_INVALID_ARG, "plan is null");
     sbr::DeviceGuard device_guard;
-    SBR_CUDA(cudaSetDevice(p->scene->device));
+    SBR_CUDA(cudaSetDevice(p->device));
     SBR_CUDA(cudaEventRecord(p->ev0, p->stream));
     if (p->use_graph && p->mode == SBR_MODE_BATCHED) {
         if (!p->graph) {
@@ -623,21 +630,22 @@ sbr_status sbr_plan_results(sbr_plan* p, sbr_result* out) {
     if (!p || !out) return fail(SBR_ERR_INVALID_ARG, "null argument");
     if (!p->executed) return fail(SBR_ERR_INVALID_ARG, "plan was not executed");
     sbr::DeviceGuard device_guard;
-    SBR_CUDA(cudaSetDevice(p->scene->device));
+    SBR_CUDA(cudaSetDevice(p->device));
     SBR_CUDA(cudaEventSynchronize(p->ev1));
-    sbr_status st = check_device_errors(p);
-    if (st != SBR_OK) return st;
     float ms = 0.0f;
     SBR_CUDA(cudaEventElapsedTime(&ms, p->ev0, p->ev1));
-    out->device_ms = ms;
     const int64_t n_out = p->n_samples * p->n_pol;
-    std::vector<double> f(2 * (size_t)n_out);
-    if (n_out)
-        SBR_CUDA(cudaMemcpyAsync(f.data(), p->d_field, f.size() * sizeof(double), cudaMemcpyDeviceToHost, p->stream));
-    if (out->stats && p->n_segs)
-        SBR_CUDA(cudaMemcpyAsync(out->stats, p->d_stats, 4 * (size_t)p->n_segs * sizeof(uint64_t),
-                                 cudaMemcpyDeviceToHost, p->stream));
+    std::vector<char> down(out->stats ? p->results_bytes : p->stats_at);
+    SBR_CUDA(cudaMemcpyAsync(down.data(), p->d_err, down.size(), cudaMemcpyDeviceToHost, p->stream));
     SBR_CUDA(cudaStreamSynchronize(p->stream));
+    uint32_t err = 0;
+    std::memcpy(&err, down.data(), sizeof(err));
+    sbr_status st = report_device_errors(p, err);
+    if (st != SBR_OK) return st;
+    out->device_ms = ms;
+    const double* f = reinterpret_cast<const double*>(down.data() + 256);
+    if (out->stats && p->n_segs)
+        std::memcpy(out->stats, down.data() + p->stats_at, 4 * (size_t)p->n_segs * sizeof(uint64_t));
     for (int64_t i = 0; i < n_out; ++i) {
         double re = f[2 * i], im = f[2 * i + 1];
         if (out->field) { out->field[2 * i] = re; out->field[2 * i + 1] = im; }
@@ -650,6 +658,7 @@ sbr_status sbr_plan_results(sbr_plan* p, sbr_result* out) {
 
 sbr_status sbr_plan_device_results(sbr_plan* p, const double** d_field, const uint64_t** d_stats) {
     if (!p) return fail(SBR_ERR_INVALID_ARG, "plan is null");
+    p->handed_out = true;
     if (d_field) *d_field = p->d_field;
     if (d_stats) *d_stats = reinterpret_cast<const uint64_t*>(p->d_stats);
     return SBR_OK;
@@ -716,7 +725,7 @@ sbr_status sbr_trace_records(sbr_scene* s, const sbr_job* job, const sbr_run_opt
     if (st != SBR_OK) return st;
     long long n = (long long)job->n_angles * job->nx * job->ny;
     sbr_ray_record* d = nullptr;
-    cudaError_t e = cudaMalloc(&d, std::max<long long>(n, 1) * sizeof(sbr_ray_record));
+    cudaError_t e = pool_alloc(p->device, &d, (size_t)n * sizeof(sbr_ray_record));
     if (e != cudaSuccess) {
         release(p);
         return fail(SBR_ERR_OOM, "record buffer allocation failed");
@@ -732,7 +741,8 @@ sbr_status sbr_trace_records(sbr_scene* s, const sbr_job* job, const sbr_run_opt
         e = cudaMemcpy(out, d, n * sizeof(sbr_ray_record), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) st = cuda_fail(e, "record copy");
     }
-    cudaFree(d);
+    cudaStreamSynchronize(p->stream);
+    pool_free(p->device, d);
     release(p);
     return st;
 }
@@ -758,8 +768,8 @@ sbr_status sbr_trace_ray_list(sbr_scene* s, const sbr_job* job, const sbr_run_op
     int32_t* d_rays = nullptr;
     sbr_ray_record* d = nullptr;
     const size_t n = std::max<size_t>(n_rays, 1);
-    cudaError_t e = cudaMalloc(&d_rays, n * 3 * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&d, n * sizeof(sbr_ray_record));
+    cudaError_t e = pool_alloc(p->device, &d_rays, n * 3 * sizeof(int32_t));
+    if (e == cudaSuccess) e = pool_alloc(p->device, &d, n * sizeof(sbr_ray_record));
     if (e != cudaSuccess) st = fail(SBR_ERR_OOM, "ray list allocation failed");
     if (st == SBR_OK && n_rays) {
         e = cudaMemcpyAsync(d_rays, rays, n_rays * 3 * sizeof(int32_t), cudaMemcpyHostToDevice, p->stream);
@@ -776,8 +786,9 @@ sbr_status sbr_trace_ray_list(sbr_scene* s, const sbr_job* job, const sbr_run_op
         e = cudaMemcpy(out, d, n_rays * sizeof(sbr_ray_record), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) st = cuda_fail(e, "record copy");
     }
-    cudaFree(d);
-    cudaFree(d_rays);
+    cudaStreamSynchronize(p->stream);
+    pool_free(p->device, d);
+    pool_free(p->device, d_rays);
     release(p);
     return st;
 }

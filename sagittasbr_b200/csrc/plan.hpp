@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "common.hpp"
+#include "devpool.hpp"
 
 struct sbr_scene {
     int device = 0;
@@ -20,7 +21,8 @@ struct sbr_scene {
     std::vector<float> xyz;          // caller vertices (unscaled)
     std::vector<uint32_t> idx;
     std::vector<int32_t> order;      // leaf slot -> caller triangle index
-    // device
+    // device: one block (nodes to d_cancel), the others apart
+    void* block = nullptr;
     sbr::GNode4* d_nodes = nullptr;
     int64_t n_gnodes = 0;
     sbr::GNode8* d_nodes8 = nullptr;  // node_width 8: the same leaves under 8-wide nodes
@@ -37,7 +39,6 @@ struct sbr_scene {
     uint32_t* d_idx = nullptr;
     uint32_t* d_err = nullptr;
     int32_t* d_cancel = nullptr;     // device word polled by the kernels
-    int32_t* h_flag_vals = nullptr;  // pinned {1, 0}: sources of the async flag copies
     cudaStream_t cancel_stream = nullptr;
     int depth = 0;
     double build_ms = 0.0;
@@ -82,7 +83,11 @@ struct sbr_plan {
     int persistent_grid = 0;
     int launches = 0;
 
-    // device
+    // device: the tables, accumulators and results in one block; the raster's buffers in
+    // another
+    int device = 0;
+    void* block = nullptr;
+    void* raster_block = nullptr;
     sbr::Segment* d_segs = nullptr;
     int64_t* d_seg_base = nullptr;
     sbr::JobConst* d_jobs = nullptr;
@@ -94,7 +99,10 @@ struct sbr_plan {
     double* d_field = nullptr;
     unsigned long long* d_stats = nullptr;
     unsigned long long* d_queue = nullptr;
-    uint32_t* d_err = nullptr;
+    uint32_t* d_err = nullptr;         // this plan's error word; the fields and counters follow it
+    bool handed_out = false;           // the caller has the results' device addresses
+    size_t results_bytes = 0;          // error word (256 bytes), d_field and d_stats: one copy
+    size_t stats_at = 0;               // of d_stats from d_err
     const volatile int32_t* d_cancel = nullptr;
     int64_t device_bytes = 0;
 

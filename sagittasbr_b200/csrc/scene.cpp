@@ -63,21 +63,11 @@ void free_scene(sbr_scene* s) {
     int cur = -1;
     cudaGetDevice(&cur);
     cudaSetDevice(s->device);
-    if (s->stream) cudaStreamSynchronize(s->stream);
-    cudaFree(s->d_nodes);
-    cudaFree(s->d_nodes8);
-    cudaFree(s->d_tris);
-    cudaFree(s->d_tris64);
-    cudaFree(s->d_tri_id);
-    cudaFree(s->d_tie);
-    cudaFree(s->d_horizon);
-    cudaFree(s->d_xyz);
-    cudaFree(s->d_idx);
-    cudaFree(s->d_refit_nodes);
-    cudaFree(s->d_tri_box);
-    cudaFree(s->d_err);
-    cudaFree(s->d_cancel);
-    if (s->h_flag_vals) cudaFreeHost(s->h_flag_vals);
+    cudaDeviceSynchronize();  // plans on the caller's streams may still walk the scene
+    for (void* q : {s->block, (void*)s->d_nodes8, (void*)s->d_tris64, (void*)s->d_xyz, (void*)s->d_idx,
+                    (void*)s->d_refit_nodes, (void*)s->d_tri_box})
+        pool_free(s->device, q);
+    pool_close(s->device);
     if (s->cancel_stream) cudaStreamDestroy(s->cancel_stream);
     if (s->stream) cudaStreamDestroy(s->stream);
     if (cur >= 0) cudaSetDevice(cur);
@@ -109,8 +99,8 @@ sbr_status ensure_fp64(sbr_scene* s) {
     sbr::DeviceGuard device_guard;
     SBR_CUDA(cudaSetDevice(s->device));
     size_t bytes = sizeof(GTri64) * t64.size();
-    cudaError_t e = cudaMalloc(&s->d_tris64, bytes);
-    if (e != cudaSuccess) return fail(SBR_ERR_OOM, "cudaMalloc of FP64 triangles failed");
+    cudaError_t e = pool_alloc(s->device, &s->d_tris64, bytes);
+    if (e != cudaSuccess) return fail(SBR_ERR_OOM, "allocation of FP64 triangles failed");
     SBR_CUDA(cudaMemcpy(s->d_tris64, t64.data(), bytes, cudaMemcpyHostToDevice));
     s->device_bytes += (int64_t)bytes;
     return SBR_OK;
@@ -143,16 +133,18 @@ sbr_status sbr_scene_create(const float* xyz, size_t nverts, const uint32_t* tri
     int dev = o.device;
     if (dev < 0) SBR_CUDA(cudaGetDevice(&dev));
     if (dev >= ndev) return fail(SBR_ERR_INVALID_ARG, "device ordinal out of range");
-    cudaDeviceProp prop;
-    SBR_CUDA(cudaGetDeviceProperties(&prop, dev));
-    if (prop.major < 10) return fail(SBR_ERR_NO_DEVICE, "libsbr is built for sm_100a (B200); device is older");
+    int major = 0, num_sms = 0;
+    SBR_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
+    SBR_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
+    if (major < 10) return fail(SBR_ERR_NO_DEVICE, "libsbr is built for sm_100a (B200); device is older");
     sbr::DeviceGuard device_guard;
     SBR_CUDA(cudaSetDevice(dev));
 
     auto t0 = std::chrono::steady_clock::now();
     sbr_scene* s = new sbr_scene();
     s->device = dev;
-    s->num_sms = prop.multiProcessorCount;
+    pool_open(dev);
+    s->num_sms = num_sms;
     s->ntris = (int64_t)ntris;
     s->model_scale = scale;
     s->xyz.assign(xyz, xyz + 3 * nverts);
@@ -397,51 +389,46 @@ sbr_status sbr_scene_create(const float* xyz, size_t nverts, const uint32_t* tri
         return st;
     };
     cudaError_t e;
-    size_t nb = sizeof(GNode4) * g.size(), tb = sizeof(GTri) * tr.size(), ib = sizeof(int32_t) * ids.size();
-    if ((e = cudaMalloc(&s->d_nodes, nb)) != cudaSuccess || (e = cudaMalloc(&s->d_tris, tb)) != cudaSuccess ||
-        (e = cudaMalloc(&s->d_tri_id, ib)) != cudaSuccess || (e = cudaMalloc(&s->d_err, sizeof(uint32_t))) != cudaSuccess)
+    const size_t nb = sizeof(GNode4) * g.size(), tb = sizeof(GTri) * tr.size(), ib = sizeof(int32_t) * ids.size(),
+                 hb = sizeof(unsigned long long) * ntris, rb = sizeof(int32_t) * tie.size();
+    Parts parts;
+    const size_t node_at = parts.add(nb), tri_at = parts.add(tb), id_at = parts.add(ib), hor_at = parts.add(hb),
+                 tie_at = parts.add(rb), err_at = parts.add(sizeof(uint32_t)), cancel_at = parts.add(sizeof(int32_t));
+    char* b = nullptr;
+    if ((e = pool_alloc(dev, &b, parts.size())) != cudaSuccess)
         return bail(fail(SBR_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(e)));
-    if ((e = cudaMemcpy(s->d_nodes, g.data(), nb, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(s->d_tris, tr.data(), tb, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(s->d_tri_id, ids.data(), ib, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = clear_device_word(s->d_err)) != cudaSuccess)
-        return bail(cuda_fail(e, "scene upload"));
-    // cancel flag: a device word (the kernels poll it from L2); the host sets it with an
-    // asynchronous copy on a side stream, which runs while the sweep kernel is resident
-    if ((e = cudaMalloc(&s->d_cancel, sizeof(int32_t))) != cudaSuccess ||
-        (e = clear_device_word(s->d_cancel)) != cudaSuccess)
-        return bail(cuda_fail(e, "cancel flag"));
-    if ((e = cudaHostAlloc(&s->h_flag_vals, 2 * sizeof(int32_t), cudaHostAllocDefault)) != cudaSuccess)
-        return bail(cuda_fail(e, "cudaHostAlloc(cancel values)"));
-    s->h_flag_vals[0] = 1;
-    s->h_flag_vals[1] = 0;
+    s->block = b;
+    s->d_nodes = reinterpret_cast<GNode4*>(b + node_at);
+    s->d_tris = reinterpret_cast<GTri*>(b + tri_at);
+    s->d_tri_id = reinterpret_cast<int32_t*>(b + id_at);
+    s->d_horizon = reinterpret_cast<unsigned long long*>(b + hor_at);
+    if (rb) s->d_tie = reinterpret_cast<int32_t*>(b + tie_at);
+    s->d_err = reinterpret_cast<uint32_t*>(b + err_at);
+    // cancel flag: a device word (the kernels poll it from L2); the host sets it on a side
+    // stream, which runs while the sweep kernel is resident
+    s->d_cancel = reinterpret_cast<int32_t*>(b + cancel_at);
     if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&s->cancel_stream, cudaStreamNonBlocking)) != cudaSuccess)
         return bail(cuda_fail(e, "cudaStreamCreate"));
-    s->device_bytes = (int64_t)(nb + tb + ib);
-    if (!tie.empty()) {
-        if ((e = cudaMalloc(&s->d_tie, ib)) != cudaSuccess)
-            return bail(fail(SBR_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(e)));
-        if ((e = cudaMemcpy(s->d_tie, tie.data(), ib, cudaMemcpyHostToDevice)) != cudaSuccess)
-            return bail(cuda_fail(e, "tie rank upload"));
-        s->device_bytes += (int64_t)ib;
-    }
+    if ((e = cudaMemcpyAsync(s->d_nodes, g.data(), nb, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(s->d_tris, tr.data(), tb, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(s->d_tri_id, ids.data(), ib, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess ||
+        (rb && (e = cudaMemcpyAsync(s->d_tie, tie.data(), rb, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess) ||
+        (e = cudaMemsetAsync(s->d_err, 0, sizeof(uint32_t), s->stream)) != cudaSuccess ||
+        (e = cudaMemsetAsync(s->d_cancel, 0, sizeof(int32_t), s->stream)) != cudaSuccess)
+        return bail(cuda_fail(e, "scene upload"));
+    s->device_bytes = (int64_t)parts.size();
     if (!g8.empty()) {
         const size_t nb8 = sizeof(GNode8) * g8.size();
-        if ((e = cudaMalloc(&s->d_nodes8, nb8)) != cudaSuccess)
+        if ((e = pool_alloc(dev, &s->d_nodes8, nb8)) != cudaSuccess)
             return bail(fail(SBR_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(e)));
-        if ((e = cudaMemcpy(s->d_nodes8, g8.data(), nb8, cudaMemcpyHostToDevice)) != cudaSuccess)
+        if ((e = cudaMemcpyAsync(s->d_nodes8, g8.data(), nb8, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess)
             return bail(cuda_fail(e, "8-wide node upload"));
         s->device_bytes += (int64_t)nb8;
     }
-    {
-        const size_t hb = sizeof(unsigned long long) * ntris;
-        if ((e = cudaMalloc(&s->d_horizon, hb)) != cudaSuccess)
-            return bail(fail(SBR_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(e)));
-        sbr_status st = build_horizons(s);
-        if (st != SBR_OK) return bail(st);
-        s->device_bytes += (int64_t)hb;
-    }
+    // (waits for the uploads as well)
+    sbr_status hs = build_horizons(s);
+    if (hs != SBR_OK) return bail(hs);
     if (o.want_fp64 > 0) {
         sbr_status st = ensure_fp64(s);
         if (st != SBR_OK) return bail(st);
@@ -474,8 +461,7 @@ sbr_status sbr_scene_cancel(sbr_scene* s) {
     if (!s) return fail(SBR_ERR_INVALID_ARG, "scene is null");
     sbr::DeviceGuard device_guard;
     SBR_CUDA(cudaSetDevice(s->device));
-    SBR_CUDA(cudaMemcpyAsync(s->d_cancel, &s->h_flag_vals[0], sizeof(int32_t), cudaMemcpyHostToDevice,
-                             s->cancel_stream));
+    SBR_CUDA(cudaMemsetAsync(s->d_cancel, 1, sizeof(int32_t), s->cancel_stream));
     return SBR_OK;
 }
 
@@ -483,8 +469,7 @@ sbr_status sbr_scene_reset_cancel(sbr_scene* s) {
     if (!s) return fail(SBR_ERR_INVALID_ARG, "scene is null");
     sbr::DeviceGuard device_guard;
     SBR_CUDA(cudaSetDevice(s->device));
-    SBR_CUDA(cudaMemcpyAsync(s->d_cancel, &s->h_flag_vals[1], sizeof(int32_t), cudaMemcpyHostToDevice,
-                             s->cancel_stream));
+    SBR_CUDA(cudaMemsetAsync(s->d_cancel, 0, sizeof(int32_t), s->cancel_stream));
     SBR_CUDA(cudaStreamSynchronize(s->cancel_stream));
     return SBR_OK;
 }
