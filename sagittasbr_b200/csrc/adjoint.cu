@@ -216,8 +216,9 @@ __global__ void __launch_bounds__(kCtaThreads, 6) k_adjoint(const AdjointParams 
         const FreqConst* F = P.freqs + J.freq_base;
         const double* cot = P.cot + 2 * G.sample_base;
         for (int k = 0; k < K; ++k) gk[k] = 0.0;
-        const int b0 = int(item - G.item_base) * G.blocks_per_item;
-        const int nslots = min(G.blocks_per_item, G.blocks - b0) * 32;
+        const Run run = item_run(G, item, false);
+        const int b0 = run.first;
+        const int nslots = run.count * 32;
         for (int s0 = 0; s0 < nslots; s0 += 32) {  // one 4x8 ray block per step, all lanes
             const int s = s0 + lane;
             const int blk = b0 + (s >> 5), l = s & 31;

@@ -125,6 +125,8 @@ struct __align__(16) Segment {
     int32_t blocks_x;     // ray blocks across the clipped rectangle
     int32_t blocks;       // blocks in the clipped rectangle
     int32_t blocks_per_item;
+    int32_t parts;        // work items that share a run of blocks_per_item blocks (item_run)
+    int32_t part_blocks;  // blocks of one of them
     int32_t tbase;        // first-hit raster: first tile (ray block) of this segment within its chunk
     int64_t item_base;    // first work item of this segment
     int64_t sample_base;  // first output sample (angle, freq) index

@@ -15,7 +15,7 @@ namespace sbr {
 namespace {
 
 constexpr int kDevices = 64;
-constexpr unsigned long long kKeepOpen = 1ull << 30;   // a chunk of raster buffers fits (plan.cpp)
+constexpr unsigned long long kKeepOpen = 2560ull << 20;  // a chunk of raster buffers fits (plan.cpp)
 constexpr unsigned long long kKeepIdle = 64ull << 20;
 
 struct Pool {

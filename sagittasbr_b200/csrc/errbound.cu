@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(kCtaThreads) k_errbound(const ErrParams P) {
         const FreqConst* F = P.freqs + J.freq_base;
         double kmax = 0.0;
         for (int k = 0; k < J.n_freqs; ++k) kmax = fmax(kmax, F[k].k);
-        const int b0 = int(item - G.item_base) * G.blocks_per_item;
-        const int b1 = min(b0 + G.blocks_per_item, G.blocks);
+        const Run run = item_run(G, item, false);
+        const int b0 = run.first, b1 = run.first + run.count;
         double sa = 0.0, s1 = 0.0, q1 = 0.0, s0 = 0.0, q2 = 0.0;
         unsigned nex = 0, nray = 0;
         for (int blk = b0; blk < b1; ++blk) {
@@ -459,7 +459,10 @@ extern "C" sbr_status sbr_error_bound(sbr_scene* s, const sbr_job* jobs, size_t 
         for (int64_t g = 0; g < p->n_segs; ++g) {
             const Segment& G = p->segs[(size_t)g];
             const JobConst& J = p->jobs[(size_t)G.job];
-            const int64_t items = p->seg_base[(size_t)g + 1] - p->seg_base[(size_t)g];
+            // folds of the sweep, in runs of blocks; a run's items (cut_items) round it several
+            // times, independently, by at most half a unit each
+            const int run = o.blocks_per_item > 0 ? G.blocks_per_item : auto_run(G.blocks);
+            const int64_t items = (G.blocks + run - 1) / run;
             for (int k = 0; k < J.n_freqs; ++k) {
                 const FreqConst& F = p->freqs[(size_t)(J.freq_base + k)];
                 const int64_t smp = G.sample_base + k;

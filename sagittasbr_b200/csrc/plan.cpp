@@ -244,9 +244,11 @@ sbr_status build_tables(const sbr_scene* const* scenes, const int32_t* job_scene
             // up to 8 blocks (256 rays) per warp item in batched mode, fewer when a
             // segment is small; one block per item in per-angle mode, where a single
             // segment must spread over the whole GPU
-            int bpi = o.mode == SBR_MODE_BATCHED ? std::max(1, std::min(8, g.blocks / 1024)) : 1;
+            int bpi = o.mode == SBR_MODE_BATCHED ? auto_run(g.blocks) : 1;
             if (o.blocks_per_item > 0) bpi = std::min(o.blocks_per_item, 1024);
             g.blocks_per_item = bpi;
+            g.parts = 1;
+            g.part_blocks = bpi;
             g.item_base = item;
             g.sample_base = sample;
             item += (g.blocks + bpi - 1) / bpi;
@@ -281,6 +283,34 @@ struct PlanSink : sbr::TableSink {
         return true;
     }
 };
+
+// Cuts a batched plan's automatic work items down to 1, 2, 4 or 8 blocks: a launch ends
+// when its slowest warps have finished the items they took last, and items of 8 blocks
+// with a few five-bounce rays among them run for most of a millisecond.  With few blocks
+// per resident warp that end weighs most, with many the items' own set-up and fold.  Measured on B200 (blocks per resident warp: ms at items of 1 /
+// 2 / 4 / 8 blocks): sphere (11) 0.457 / 0.476 / 0.521 / 0.564, plates (55) 2.40 / 2.47 /
+// 2.72 / 3.11, ellipsoid (65) 2.21 / 2.19 / 2.21 / 2.40, narrow aircraft (261) 2.97 / 2.77
+// / 3.15 / 3.30, HH + VV aircraft (578) 9.15 / 6.74 / 6.67 / 7.35, wideband aircraft (1570)
+// 34.7 / 24.9 / 22.8 / 23.7, its 61 azimuths (15,800) 199.5 ms at 4 and 197.2 at 8.  Sweeps with FP32 partial sums per group of rays (`groups`)
+// keep their runs of blocks, in which the groups form, and share them between items.
+void cut_items(sbr_plan* p, bool groups) {
+    int64_t blocks = 0;
+    for (const Segment& g : p->segs) blocks += g.blocks;
+    const int64_t per_warp = blocks / (int64_t(32) * p->num_sms);
+    const int32_t most = per_warp < 32 ? 1 : per_warp < 512 ? 2 : per_warp < 2048 ? 4 : 8;
+    int64_t item = 0;
+    for (size_t k = 0; k < p->segs.size(); ++k) {
+        Segment& g = p->segs[k];
+        const int32_t n = std::min(most, g.blocks_per_item);
+        if (!groups) g.blocks_per_item = n;
+        g.part_blocks = n;
+        g.parts = (g.blocks_per_item + n - 1) / n;
+        g.item_base = item;
+        item += (int64_t)((g.blocks + g.blocks_per_item - 1) / g.blocks_per_item) * g.parts;
+        p->seg_base[k + 1] = item;
+    }
+    p->n_items = item;
+}
 
 }  // namespace
 
@@ -423,6 +453,8 @@ sbr_status plan_create(sbr_scene* const* scenes, size_t n_scenes, const int32_t*
     p->n_rays_clipped = tot.n_rays_clipped;
     p->n_rays_grid = tot.n_rays_grid;
     p->n_pol = p->pol == SBR_POL_HHVV ? 2 : 1;
+    if (o.mode == SBR_MODE_BATCHED && o.blocks_per_item == 0)
+        cut_items(p, o.precision == SBR_PREC_MIXED && p->k_max * p->n_pol > max_lane_channels());
     // a refitted scene has no horizons: a plan that launches enough rays to pay for them
     // (5 to 20 ns a triangle against 50 to 100 ps a ray, measured on B200) brings them back
     if (!p->multi && p->prec != SBR_PREC_FP32 && p->n_rays_clipped >= 200 * s->ntris) {
@@ -463,19 +495,19 @@ sbr_status plan_create(sbr_scene* const* scenes, size_t n_scenes, const int32_t*
                 (o.first_hit == SBR_FIRST_HIT_RASTER || (o.first_hit == SBR_FIRST_HIT_AUTO && dense));
     if (p->raster) {
         // per tile: 32 first-hit entries (8 B), a count and `cap` list entries (4 B).  A
-        // chunk holds 1 GiB of them, which the memory pool keeps from one call to the next
+        // chunk holds 2.5 GiB of them, which the memory pool keeps from one call to the next
         // (a 181-azimuth narrow sweep's 2.8 GB in one piece cost 2.6 ms of mapping a call),
-        // and more, up to 8 GiB, until it has 12 segments: every chunk ends with a wait for
+        // and more, up to 8 GiB, until it has 16 segments: every chunk ends with a wait for
         // its slowest warps (0.5 ms an azimuth when 10 azimuths of the 12,222^2 grid,
         // 0.55 GB each, went one by one instead of together: 44.7 against 31.9 ms).
         p->tile_cap = o.tile_cap > 0 ? (uint32_t)o.tile_cap : 48u;
         const int64_t tile_bytes = 32 * 8 + 4 + 4 * (int64_t)p->tile_cap;
-        const int64_t budget = (int64_t(1023) << 20) / tile_bytes, most = (int64_t(8) << 30) / tile_bytes;
+        const int64_t budget = (int64_t(2559) << 20) / tile_bytes, most = (int64_t(8) << 30) / tile_bytes;
         sbr_plan::Chunk c{0, 0, 0, 0, 0, 0};
         for (size_t g = 0; g < p->segs.size(); ++g) {
             const int64_t tiles = p->segs[g].blocks, held = c.seg_end - c.seg_begin;
             // (the binning launch's grid.y is the chunk's segment count: at most 65535)
-            if (held > 0 && (c.tiles + tiles > most || (c.tiles + tiles > budget && held >= 12) || held >= 65535)) {
+            if (held > 0 && (c.tiles + tiles > most || (c.tiles + tiles > budget && held >= 16) || held >= 65535)) {
                 c.item_end = p->seg_base[c.seg_end];
                 p->chunks.push_back(c);
                 c = sbr_plan::Chunk{c.seg_end, c.seg_end, p->seg_base[c.seg_end], 0, 0, 0};

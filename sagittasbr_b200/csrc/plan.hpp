@@ -151,12 +151,15 @@ sbr_status validate_run(const sbr_scene* s, const sbr_job* jobs, size_t n_jobs, 
 sbr_status build_tables(const sbr_scene* const* scenes, const int32_t* job_scene, const sbr_job* jobs,
                         size_t n_jobs, const sbr_run_opts& o, TableSink& sink, TableTotals& tot);
 
+// Blocks per work item of a segment of a batched sweep, before they are cut down.
+inline int auto_run(int blocks) { return blocks / 1024 < 1 ? 1 : blocks / 1024 > 8 ? 8 : blocks / 1024; }
 sbr_status plan_launch(sbr_plan* pl, bool records, sbr_ray_record* d_records);
 
 sbr_status fill_records(sbr_ray_record* d, long long n, cudaStream_t st);
 // Traces the listed rays (angle index, i, j; checked by the caller) of a one-job plan.
 sbr_status trace_list_launch(sbr_plan* pl, const int32_t* d_rays, long long n, sbr_ray_record* d_out);
 int max_freqs_per_job();
+int max_lane_channels();  // channels up to which every lane sums its own rays' terms
 sbr_status ensure_fp64(sbr_scene* s);
 sbr_status ensure_adjoint_data(sbr_scene* s);
 // Computes the scene's horizons unless it holds them, and waits for them.

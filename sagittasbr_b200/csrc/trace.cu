@@ -205,8 +205,9 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
         const int kb = P.k_count > 0 ? P.k_begin : 0;
         const int K = P.k_count > 0 ? P.k_count : J.n_freqs;
         const FreqConst* F = P.freqs + J.freq_base + kb;
-        const int b0 = int(item - G.item_base) * G.blocks_per_item;
-        const int nslots = min(G.blocks_per_item, G.blocks - b0) * 32;
+        const Run run = item_run(G, item, PART);
+        const int b0 = run.first;
+        const int nslots = run.count * 32;
         const int i_end = G.i0 + G.ni, j_end = G.j0 + G.nj;
         const int KC = K * NPOL;  // channels of this item
 
@@ -1011,6 +1012,7 @@ sbr_status fill_records(sbr_ray_record* d, long long n, cudaStream_t st) {
 }
 
 int max_freqs_per_job() { return kMaxK; }
+int max_lane_channels() { return kRegK; }
 
 }  // namespace sbr
 

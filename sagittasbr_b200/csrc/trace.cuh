@@ -791,6 +791,31 @@ struct Walker<true> {
     }
 };
 
+// Blocks of a work item.  Where several items share a run, each takes part_blocks of it;
+// but with `groups` (FP32 partial sums per group of 32 rays, trace.cu) a run with a
+// ragged block stays whole and goes to its first item, because the lanes a ragged block
+// leaves idle take rays of the blocks that follow it in the run.
+struct Run {
+    int first, count;
+};
+__device__ __forceinline__ Run item_run(const Segment& G, long long item, bool groups) {
+    const int k = int(item - G.item_base);
+    const int run = k / G.parts, part = k - run * G.parts;
+    Run r{run * G.blocks_per_item, 0};
+    r.count = min(G.blocks_per_item, G.blocks - r.first);
+    if (G.parts == 1) return r;
+    const bool column = (G.ni % kBlockW) != 0 && r.first % G.blocks_x + r.count >= G.blocks_x;
+    const bool row = (G.nj % kBlockH) != 0 && r.first + r.count > G.blocks - G.blocks_x;
+    if (groups && (column || row)) {
+        if (part > 0) r.count = 0;
+        return r;
+    }
+    const int lo = part * G.part_blocks;
+    r.count = max(0, min(G.part_blocks, r.count - lo));
+    r.first += lo;
+    return r;
+}
+
 // Segment owning a work item: base[] holds each segment's first item (ascending).
 __device__ __forceinline__ int find_segment(const int64_t* base, int n, int64_t item) {
     int lo = 0, hi = n;  // base[lo] <= item < base[hi]
