@@ -133,6 +133,7 @@ struct __align__(16) Segment {
     // pixel coordinates of a point P on the launcher grid: s = ps[0..2].P + ps[3],
     // t = pt[0..2].P + pt[3] (pixel (i, j) is centred at s = i, t = j)
     double ps[4], pt[4];
+    float margin;         // pixels by which the first-hit raster widens projected triangles
     int64_t zbase;        // first first-hit buffer entry of this segment within its chunk (32 tbase;
                           // entries are tile-major: tile, then lane of the 4 x 8 block)
 };

@@ -235,6 +235,12 @@ sbr_status build_tables(const sbr_scene* const* scenes, const int32_t* job_scene
             }
             g.ps[3] = -(fd.llc[0] * g.ps[0] + fd.llc[1] * g.ps[1] + fd.llc[2] * g.ps[2]) - 0.5;
             g.pt[3] = -(fd.llc[0] * g.pt[0] + fd.llc[1] * g.pt[1] + fd.llc[2] * g.pt[2]) - 0.5;
+            // the raster's margin: 0.06 pixel plus 2^-19 of the largest launcher coordinate over
+            // the pixel size, which covers the FP32 rounding of the ray origins, of the
+            // triangle test's sheared coordinates and of the edge tests
+            double ext = 0.0;
+            for (int k = 0; k < 3; ++k) ext += std::fabs(g.llc[k]) + std::fabs(g.u[k]) + std::fabs(g.v[k]);
+            g.margin = float(0.06 + std::ldexp(ext, -19) / std::min(std::sqrt(uu) / J.nx, std::sqrt(vv) / J.ny)) * 1.000001f;
             g.zbase = 0;
             g.job = (int32_t)j;
             g.angle = (int32_t)a;

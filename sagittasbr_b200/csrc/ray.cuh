@@ -131,15 +131,18 @@ constexpr unsigned long long kZMiss = ~0ull;
 constexpr unsigned long long kZWalk = 0xfffffffe00000000ull;
 
 // One closest-hit query, then reflect and nudge; true when the ray is finished.
-// The first query is read from the first-hit buffer when there is one.
+// The first query is read from the first-hit buffer when there is one (a tile no
+// triangle reaches has no entries there).
 // SPEC: the speculative closest-hit walk, entered by all lanes of `mask` together.
 template <int PREC, bool REC, bool POL, bool W8 = false, bool SPEC = false>
 __device__ __forceinline__ bool step_f(RayF& r, PolF& e, const SceneView& S, int maxB, uint32_t& err,
-                                       sbr_ray_record* rec, unsigned long long* zbuf, unsigned mask = 0u) {
+                                       sbr_ray_record* rec, const unsigned long long* zbuf, const uint32_t* tile_cnt,
+                                       unsigned mask = 0u) {
     if (PREC == SBR_PREC_MIXED && r.zidx < 0) return true;
     float tB = 1e20f;
     int slot;
-    const unsigned long long key = (zbuf != nullptr && r.count == 0) ? zbuf[r.zidx] : kZWalk;
+    unsigned long long key = kZWalk;
+    if (zbuf != nullptr && r.count == 0) key = tile_cnt[r.zidx >> 5] == 0u ? kZMiss : zbuf[r.zidx];
     if (key == kZMiss) return true;
     if (key != kZWalk) {
         tB = __uint_as_float((unsigned)(key >> 32));
