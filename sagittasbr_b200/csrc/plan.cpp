@@ -62,12 +62,15 @@ void release(sbr_plan* p) {
     sbr::DeviceGuard device_guard;
     cudaSetDevice(p->device);
     // the blocks go back to the pool: nothing may use them any more
-    if (p->handed_out || (p->stream && cudaStreamSynchronize(p->stream) != cudaSuccess)) cudaDeviceSynchronize();
+    if (p->handed_out || p->forked || (p->stream && cudaStreamSynchronize(p->stream) != cudaSuccess)) cudaDeviceSynchronize();
     if (p->graph) cudaGraphExecDestroy(p->graph);
     pool_free(p->device, p->block);
     pool_free(p->device, p->raster_block);
     if (p->ev0) cudaEventDestroy(p->ev0);
     if (p->ev1) cudaEventDestroy(p->ev1);
+    if (p->fork) cudaEventDestroy(p->fork);
+    for (cudaEvent_t e : p->join)
+        if (e) cudaEventDestroy(e);
     delete p;
 }
 
@@ -88,6 +91,36 @@ sbr_status check_device_errors(sbr_plan* p) {
 }  // namespace
 
 namespace sbr {
+
+sbr_status plan_fork(sbr_plan* p) {
+    sbr_scene* s = p->scene;
+    if (!p->side) {
+        int64_t launches = 0;
+        for (size_t g = 0; g < p->segs.size() && launches < kSideStreams; ++g)
+            if (p->seg_base[g + 1] > p->seg_base[g]) launches += p->jobs[p->segs[g].job].n_freqs;
+        p->n_side = (int)std::min<int64_t>(launches, kSideStreams);
+        std::lock_guard<std::mutex> lock(s->side_mu);
+        SBR_CUDA(cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming));
+        for (int k = 0; k < p->n_side; ++k) {
+            if (!s->side[k]) SBR_CUDA(cudaStreamCreateWithFlags(&s->side[k], cudaStreamNonBlocking));
+            SBR_CUDA(cudaEventCreateWithFlags(&p->join[k], cudaEventDisableTiming));
+        }
+        p->side = s->side;
+    }
+    p->forked = true;
+    SBR_CUDA(cudaEventRecord(p->fork, p->stream));
+    for (int k = 0; k < p->n_side; ++k) SBR_CUDA(cudaStreamWaitEvent(p->side[k], p->fork, 0));
+    return SBR_OK;
+}
+
+sbr_status plan_join(sbr_plan* p) {
+    for (int k = 0; k < p->n_side; ++k) {
+        SBR_CUDA(cudaEventRecord(p->join[k], p->side[k]));
+        SBR_CUDA(cudaStreamWaitEvent(p->stream, p->join[k], 0));
+    }
+    p->forked = false;
+    return SBR_OK;
+}
 
 sbr_status validate_run(const sbr_scene* s, const sbr_job* jobs, size_t n_jobs, const sbr_run_opts& o) {
     if (!s || (!jobs && n_jobs)) return fail(SBR_ERR_INVALID_ARG, "null scene or jobs");

@@ -69,6 +69,8 @@ void free_scene(sbr_scene* s) {
         pool_free(s->device, q);
     pool_close(s->device);
     if (s->cancel_stream) cudaStreamDestroy(s->cancel_stream);
+    for (cudaStream_t q : s->side)
+        if (q) cudaStreamDestroy(q);
     if (s->stream) cudaStreamDestroy(s->stream);
     if (cur >= 0) cudaSetDevice(cur);
     delete s;
