@@ -258,20 +258,6 @@ struct AdjointBuffers {
 
 }  // namespace
 
-// Caller vertices and triangles on the device (uploaded once per scene).
-sbr_status ensure_adjoint_data(sbr_scene* s) {
-    if (s->d_xyz && s->d_idx) return SBR_OK;
-    sbr::DeviceGuard device_guard;
-    SBR_CUDA(cudaSetDevice(s->device));
-    const size_t vb = s->xyz.size() * sizeof(float), ib = s->idx.size() * sizeof(uint32_t);
-    if (pool_alloc(s->device, &s->d_xyz, vb) != cudaSuccess || pool_alloc(s->device, &s->d_idx, ib) != cudaSuccess)
-        return fail(SBR_ERR_OOM, "allocation of the adjoint mesh copy failed");
-    SBR_CUDA(cudaMemcpy(s->d_xyz, s->xyz.data(), vb, cudaMemcpyHostToDevice));
-    SBR_CUDA(cudaMemcpy(s->d_idx, s->idx.data(), ib, cudaMemcpyHostToDevice));
-    s->device_bytes += (int64_t)(vb + ib);
-    return SBR_OK;
-}
-
 }  // namespace sbr
 
 extern "C" sbr_status sbr_adjoint(sbr_scene* s, const sbr_job* jobs, size_t n_jobs, const sbr_run_opts* opts,
@@ -296,9 +282,8 @@ extern "C" sbr_status sbr_adjoint(sbr_scene* s, const sbr_job* jobs, size_t n_jo
     } guard{p};
     for (int64_t g = 0; g < p->n_segs; ++g)
         if (p->jobs[p->segs[g].job].n_freqs > kAdjMaxK) return fail(SBR_ERR_TOO_LARGE, "more than 128 frequencies");
-    if ((st = ensure_adjoint_data(s)) != SBR_OK) return st;
 
-    const size_t nv3 = s->xyz.size(), ns = (size_t)p->n_samples;
+    const size_t nv3 = 3 * (size_t)s->nverts, ns = (size_t)p->n_samples;
     cudaStream_t stream = p->stream;
     AdjointBuffers B{s->device, stream};
     Parts parts;

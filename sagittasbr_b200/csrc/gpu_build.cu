@@ -16,9 +16,17 @@
 // Per level: big nodes (more than kWarpMax triangles) get their bounds and bins from
 // grid-wide atomics (warp-aggregated), small nodes one warp each with bins in shared
 // memory; then flags, one exclusive scan over all positions, a stable scatter, and
-// child allocation.  Nodes are numbered breadth first on the device and renumbered
-// in pre-order on the host.  One device-to-host read per level (the next level's
-// node count); no kernel waits on another.
+// child allocation.  Nodes are numbered breadth first on the device.  One
+// device-to-host read per level (the next level's node count); no kernel waits on
+// another.
+//
+// The rest of a scene's set-up runs here too: triangle boxes and centroids before the
+// build, the collapse to 4-wide nodes after it (one pass down that opens children, one up
+// that counts subtrees, one down that numbers and writes the nodes depth first, as the
+// host's collapse does), and the search for coincident faces of opposite winding.  On the
+// host they took three quarters of a set-up with a GPU-built tree: 133k triangles, boxes
+// 1.7, transfers 2.3, renumbering 5.5, collapse 3.3, triangle records 4.1 and the search
+// 9.7 of 30 ms.
 #include <algorithm>
 #include <cfloat>
 #include <vector>
@@ -448,19 +456,258 @@ __global__ void k_assign(Work W, Level L) {
     W.node_of[p] = c < 0 ? -1 : (p < L.s[j] + L.left_count[j] ? c : c + 1);
 }
 
+// Conservative boxes of the triangles (covering the FP32 and the outward-rounded FP64
+// vertices) and their centroids, in the host build's arithmetic.
+__global__ void k_boxes(const float* __restrict__ xyz, const uint32_t* __restrict__ idx, int n, float sc32, double sc,
+                        float* __restrict__ lo, float* __restrict__ hi, float* __restrict__ cen) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    float l[3] = {INFINITY, INFINITY, INFINITY}, h[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int c = 0; c < 3; ++c) {
+        const size_t v = idx[3 * (size_t)t + c];
+        for (int a = 0; a < 3; ++a) {
+            const float x = xyz[3 * v + a], p = __fmul_rn(x, sc32);
+            const double q = __dmul_rn(double(x), sc);
+            l[a] = fminf(l[a], fminf(p, __double2float_rd(q)));
+            h[a] = fmaxf(h[a], fmaxf(p, __double2float_ru(q)));
+        }
+    }
+    for (int a = 0; a < 3; ++a) {
+        lo[3 * (size_t)t + a] = l[a];
+        hi[3 * (size_t)t + a] = h[a];
+        cen[3 * (size_t)t + a] = __fmul_rn(0.5f, __fadd_rn(l[a], h[a]));
+    }
+}
+
+// ------------------------------------------------------------------ collapse
+// Work arrays of the collapse, by breadth-first number of the 4-wide node.
+struct Collapse {
+    int32_t* bin;      // binary node it stands for
+    int32_t* need;     // stack entries a walker may hold on arrival
+    int4* kids;        // binary nodes of its children, -1 for none
+    int32_t* child;    // number of its first inner child
+    int32_t* size;     // 4-wide nodes of its subtree
+    int32_t* pre;      // 4-wide nodes allotted before it in depth-first order
+    int32_t* slot;     // its final number
+    int32_t* off;      // [levels + 2] first number of each level
+    int32_t* tail;     // nodes so far
+};
+struct BinView {
+    const float* lo;
+    const float* hi;
+    const int32_t* left;
+    const int32_t* right;
+    const int32_t* first;
+    const int32_t* count;
+};
+
+__device__ __forceinline__ float box_area(const BinView& B, int b) {
+    const float x = __fsub_rn(B.hi[3 * b], B.lo[3 * b]), y = __fsub_rn(B.hi[3 * b + 1], B.lo[3 * b + 1]),
+                z = __fsub_rn(B.hi[3 * b + 2], B.lo[3 * b + 2]);
+    return __fadd_rn(__fadd_rn(__fmul_rn(x, y), __fmul_rn(y, z)), __fmul_rn(z, x));
+}
+
+__global__ void k_collapse_root(Collapse C) {
+    C.bin[0] = 0;
+    C.need[0] = 0;
+    C.off[0] = 0;
+    C.off[1] = 1;
+    *C.tail = 1;
+}
+// A 4-wide node takes a binary node's two children and keeps opening its largest (by
+// surface area) inner child until it holds four or the walker's stack bound is reached.
+__global__ void k_collapse_open(BinView B, Collapse C, int level, int stack_depth) {
+    for (int i = C.off[level] + blockIdx.x * blockDim.x + threadIdx.x; i < C.off[level + 1]; i += gridDim.x * blockDim.x) {
+        const int b = C.bin[i], need = C.need[i];
+        int kid[4] = {b, -1, -1, -1};
+        int nk = 1;
+        if (B.left[b] >= 0) {
+            kid[0] = B.left[b];
+            kid[1] = B.right[b];
+            nk = 2;
+            while (nk < 4 && need + nk <= stack_depth) {
+                int best = -1;
+                float ba = -1.0f;
+                for (int k = 0; k < nk; ++k) {
+                    if (B.left[kid[k]] < 0) continue;
+                    const float a = box_area(B, kid[k]);
+                    if (a > ba) {
+                        ba = a;
+                        best = k;
+                    }
+                }
+                if (best < 0) break;
+                const int open = kid[best];
+                for (int k = nk; k > best + 1; --k) kid[k] = kid[k - 1];
+                kid[best] = B.left[open];
+                kid[best + 1] = B.right[open];
+                ++nk;
+            }
+        }
+        int ni = 0;
+        for (int k = 0; k < nk; ++k) ni += kid[k] != b && B.left[kid[k]] >= 0;
+        int at = ni ? atomicAdd(C.tail, ni) : 0;
+        C.kids[i] = make_int4(kid[0], kid[1], kid[2], kid[3]);
+        C.child[i] = at;
+        for (int k = 0; k < nk; ++k) {
+            if (kid[k] == b || B.left[kid[k]] < 0) continue;
+            C.bin[at] = kid[k];
+            C.need[at] = need + nk - 1;
+            ++at;
+        }
+    }
+}
+__global__ void k_collapse_level(Collapse C, int level) { C.off[level + 2] = *C.tail; }
+
+__device__ __forceinline__ bool is_inner(const BinView& B, const Collapse& C, int i, int kid) {
+    return kid >= 0 && kid != C.bin[i] && B.left[kid] >= 0;
+}
+__global__ void k_collapse_size(BinView B, Collapse C, int level) {
+    for (int i = C.off[level] + blockIdx.x * blockDim.x + threadIdx.x; i < C.off[level + 1]; i += gridDim.x * blockDim.x) {
+        const int4 q = C.kids[i];
+        const int kid[4] = {q.x, q.y, q.z, q.w};
+        int at = C.child[i], n = 1;
+        for (int k = 0; k < 4; ++k)
+            if (is_inner(B, C, i, kid[k])) n += C.size[at++];
+        C.size[i] = n;
+    }
+}
+// Numbers a node's inner children next to one another after all nodes that come before
+// it depth first, and writes the node.
+__global__ void k_collapse_emit(BinView B, Collapse C, int level, GNode4* nodes, int32_t* level_nodes) {
+    for (int i = C.off[level] + blockIdx.x * blockDim.x + threadIdx.x; i < C.off[level + 1]; i += gridDim.x * blockDim.x) {
+        const int pre = level == 0 ? 0 : C.pre[i], slot = level == 0 ? 0 : C.slot[i];
+        const int4 q = C.kids[i];
+        const int kid[4] = {q.x, q.y, q.z, q.w};
+        GNode4 N;
+        int ni = 0;
+        for (int k = 0; k < 4; ++k) ni += is_inner(B, C, i, kid[k]);
+        int at = C.child[i], num = 1 + pre, before = pre + ni;
+        for (int k = 0; k < 4; ++k) {
+            float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {1e30f, 1e30f, 1e30f};  // an empty slot's far box
+            int ref = ~0;
+            if (kid[k] >= 0) {
+                for (int a = 0; a < 3; ++a) {
+                    lo[a] = B.lo[3 * kid[k] + a];
+                    hi[a] = B.hi[3 * kid[k] + a];
+                }
+                if (is_inner(B, C, i, kid[k])) {
+                    ref = num;
+                    C.slot[at] = num++;
+                    C.pre[at] = before;
+                    before += C.size[at] - 1;
+                    ++at;
+                } else {
+                    ref = ~(B.first[kid[k]] * 16 + B.count[kid[k]]);
+                }
+            }
+            (&N.lox.x)[k] = lo[0]; (&N.hix.x)[k] = hi[0];
+            (&N.loy.x)[k] = lo[1]; (&N.hiy.x)[k] = hi[1];
+            (&N.loz.x)[k] = lo[2]; (&N.hiz.x)[k] = hi[2];
+            (&N.child.x)[k] = ref;
+        }
+        nodes[slot] = N;
+        level_nodes[i] = slot;
+    }
+}
+
+// ------------------------------------------------------------------ twins
+// A triangle's three vertices in the order of their bits, and the parity of that order
+// (-1: a repeated vertex), as has_opposed_twins compares them.
+struct TwinKey {
+    uint32_t v[9];
+    int parity;
+};
+__device__ TwinKey twin_key(const float* xyz, const uint32_t* idx, size_t t) {
+    uint32_t p[3][3];
+    for (int c = 0; c < 3; ++c)
+        for (int a = 0; a < 3; ++a) p[c][a] = __float_as_uint(xyz[3 * (size_t)idx[3 * t + c] + a]);
+    int swaps = 0;
+    auto order = [&](int a, int b) {  // p[a] before p[b]
+        const bool less = p[b][0] != p[a][0] ? p[b][0] < p[a][0] : p[b][1] != p[a][1] ? p[b][1] < p[a][1] : p[b][2] < p[a][2];
+        if (!less) return;
+        ++swaps;
+        for (int k = 0; k < 3; ++k) {
+            const uint32_t x = p[a][k];
+            p[a][k] = p[b][k];
+            p[b][k] = x;
+        }
+    };
+    order(0, 1);
+    order(1, 2);
+    order(0, 1);
+    TwinKey key;
+    bool r01 = true, r12 = true;
+    for (int k = 0; k < 3; ++k) {
+        key.v[k] = p[0][k];
+        key.v[3 + k] = p[1][k];
+        key.v[6 + k] = p[2][k];
+        r01 = r01 && p[0][k] == p[1][k];
+        r12 = r12 && p[1][k] == p[2][k];
+    }
+    key.parity = r01 || r12 ? -1 : swaps & 1;
+    return key;
+}
+// Open addressing: every distinct key keeps the first triangle that came with it; a later
+// one of the other parity is a twin.
+__global__ void k_twins(const float* __restrict__ xyz, const uint32_t* __restrict__ idx, int n, int32_t* table,
+                        uint32_t mask, int32_t* flag) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const TwinKey key = twin_key(xyz, idx, t);
+    if (key.parity < 0) return;
+    uint32_t h = 2166136261u;
+    for (int k = 0; k < 9; ++k) h = (h ^ key.v[k]) * 16777619u;
+    h ^= h >> 15;
+    h *= 0x2c1b3c6du;
+    h ^= h >> 12;
+    for (uint32_t probe = 0; probe <= mask; ++probe) {
+        const int other = atomicCAS(table + ((h + probe) & mask), -1, t);
+        if (other == -1) return;
+        const TwinKey o = twin_key(xyz, idx, other);
+        bool same = true;
+        for (int k = 0; k < 9; ++k) same = same && o.v[k] == key.v[k];
+        if (same) {
+            if (o.parity != key.parity) *flag = 1;
+            return;
+        }
+    }
+}
+
 }  // namespace
 
-// See bvh_build.hpp.  Returns false (with the CUDA error in *err) if a CUDA call fails.
-bool build_sah_gpu(const std::vector<float>& tri_lo, const std::vector<float>& tri_hi, const BuildOptions& opt,
-                   cudaStream_t stream, BinTree& out, cudaError_t* err) {
-    out = BinTree();
-    const int n = (int)(tri_lo.size() / 3);
-    if (n == 0) return true;
+size_t gpu_twins_table(size_t n) {
+    size_t m = 64;
+    while (m < 2 * n) m *= 2;
+    return m;
+}
+
+cudaError_t gpu_opposed_twins(const float* d_xyz, const uint32_t* d_idx, size_t n, int32_t* table, int32_t* d_flag,
+                              cudaStream_t stream) {
+    const size_t m = gpu_twins_table(n);
+    cudaError_t e = cudaMemsetAsync(table, 0xff, m * sizeof(int32_t), stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_flag, 0, sizeof(int32_t), stream);
+    if (e != cudaSuccess) return e;
+    k_twins<<<(unsigned)((n + 127) / 128), 128, 0, stream>>>(d_xyz, d_idx, (int)n, table, (uint32_t)(m - 1), d_flag);
+    return cudaGetLastError();
+}
+
+void gpu_tree_free(GpuTree& t, cudaStream_t stream) {
+    if (!t.block) return;
+    if (cudaStreamSynchronize(stream) != cudaSuccess) cudaDeviceSynchronize();
+    pool_free(t.device, t.block);
+    pool_free(t.device, t.level_off);
+    t.block = nullptr;
+    t.level_off = nullptr;
+}
+
+cudaError_t gpu_tree_build(const float* d_xyz, const uint32_t* d_idx, int n, double scale, const BuildOptions& opt,
+                           cudaStream_t stream, GpuTree& out) {
+    out = GpuTree();
+    out.n = n;
     const int B = std::min(std::max(2, opt.bin_count), kMaxBins);
     const int cap = std::min(n, 2 * (n / (opt.leaf_size + 1)) + 2);
     const int nblk = (n + kScanBlock - 1) / kScanBlock;
-    std::vector<float> cen(3 * (size_t)n);
-    for (size_t i = 0; i < 3 * (size_t)n; ++i) cen[i] = 0.5f * (tri_lo[i] + tri_hi[i]);
 
     Work W{};
     Level L[2]{};
@@ -500,15 +747,12 @@ bool build_sah_gpu(const std::vector<float>& tri_lo, const std::vector<float>& t
         A(&l.left_count, cap);
         A(&l.child_slot, cap);
     }
-    int device = 0;
-    char* block = nullptr;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = pool_alloc(device, &block, parts.size());
-    if (e != cudaSuccess) {
-        *err = e;
-        return false;
-    }
-    for (auto& o : owned) *o.first = block + o.second;
+    // the collapse's work: a binary tree of n leaves at most has n - 1 inner nodes
+    A(&out.work, 10 * (size_t)n);
+    cudaError_t e = cudaGetDevice(&out.device);
+    if (e == cudaSuccess) e = pool_alloc(out.device, &out.block, parts.size());
+    if (e != cudaSuccess) return e;
+    for (auto& o : owned) *o.first = out.block + o.second;
     W.lo = lo;
     W.hi = hi;
     W.cen = ce;
@@ -516,21 +760,10 @@ bool build_sah_gpu(const std::vector<float>& tri_lo, const std::vector<float>& t
     W.bins = B;
     W.leaf_size = opt.leaf_size;
     W.max_leaf = opt.max_leaf;
-    auto cleanup = [&]() {
-        if (cudaStreamSynchronize(stream) != cudaSuccess) cudaDeviceSynchronize();
-        pool_free(device, block);
-    };
-    if (e == cudaSuccess) e = cudaMemcpyAsync(lo, tri_lo.data(), 12 * (size_t)n, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hi, tri_hi.data(), 12 * (size_t)n, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ce, cen.data(), 12 * (size_t)n, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(W.counters, 0, 4 * sizeof(int32_t), stream);
-    if (e != cudaSuccess) {
-        cleanup();
-        *err = e;
-        return false;
-    }
+    e = cudaMemsetAsync(W.counters, 0, 4 * sizeof(int32_t), stream);
     const int TB = 256;
     const int gp = (n + TB - 1) / TB;
+    k_boxes<<<gp, TB, 0, stream>>>(d_xyz, d_idx, n, float(scale), scale, lo, hi, ce);
     k_init<<<gp, TB, 0, stream>>>(W, L[0]);
     const size_t bin_bytes = (size_t)3 * B * kKeys * sizeof(unsigned);
     int nact = 1, cur = 0;
@@ -557,37 +790,98 @@ bool build_sah_gpu(const std::vector<float>& tri_lo, const std::vector<float>& t
         if (e == cudaSuccess) e = cudaGetLastError();
         // cannot happen: each split node has more than leaf_size triangles
         if (e == cudaSuccess && (cnt[3] != 0 || cnt[1] > cap)) e = cudaErrorInvalidValue;
-        const int next = cnt[1];
-        nact = next;
+        nact = cnt[1];
+        out.nnodes = cnt[2];
+        ++out.levels;
         cur ^= 1;
     }
-    int nnodes = 0;
-    std::vector<int32_t> order(n);
-    if (e == cudaSuccess) e = cudaMemcpy(&nnodes, W.counters + 2, sizeof(int32_t), cudaMemcpyDeviceToHost);
-    std::vector<float> nlo, nhi;
-    std::vector<int32_t> nl, nr, nf, nc;
-    if (e == cudaSuccess) {
-        nlo.resize(3 * (size_t)nnodes);
-        nhi.resize(3 * (size_t)nnodes);
-        nl.resize(nnodes);
-        nr.resize(nnodes);
-        nf.resize(nnodes);
-        nc.resize(nnodes);
-        e = cudaMemcpy(nlo.data(), W.nlo, 12 * (size_t)nnodes, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(nhi.data(), W.nhi, 12 * (size_t)nnodes, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(nl.data(), W.nleft, 4 * (size_t)nnodes, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(nr.data(), W.nright, 4 * (size_t)nnodes, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(nf.data(), W.nfirst, 4 * (size_t)nnodes, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(nc.data(), W.ncount, 4 * (size_t)nnodes, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(order.data(), W.idx, 4 * (size_t)n, cudaMemcpyDeviceToHost);
-    }
-    cleanup();
     if (e != cudaSuccess) {
-        *err = e;
-        return false;
+        gpu_tree_free(out, stream);
+        return e;
     }
+    out.lo = W.nlo;
+    out.hi = W.nhi;
+    out.left = W.nleft;
+    out.right = W.nright;
+    out.first = W.nfirst;
+    out.count = W.ncount;
+    out.order = W.idx;
+    return cudaSuccess;
+}
+
+namespace {
+
+// The collapse's arrays in the tree's block: `work` is 10 words per triangle and a tree
+// has fewer inner nodes (4-wide nodes) than triangles, but at least one node.
+Collapse collapse_view(const GpuTree& t) {
+    const size_t m = std::max(1, t.n);
+    Collapse C;
+    C.kids = reinterpret_cast<int4*>(t.work);
+    C.bin = t.work + 4 * m;
+    C.need = t.work + 5 * m;
+    C.child = t.work + 6 * m;
+    C.size = t.work + 7 * m;
+    C.pre = t.work + 8 * m;
+    C.slot = t.work + 9 * m;
+    C.off = t.level_off;
+    C.tail = t.level_off + t.levels + 2;
+    return C;
+}
+BinView bin_view(const GpuTree& t) { return {t.lo, t.hi, t.left, t.right, t.first, t.count}; }
+constexpr int kCollapseGrid = 592;  // 4 blocks of 128 per SM, striding over a level
+
+}  // namespace
+
+cudaError_t gpu_tree_collapse(GpuTree& t, int stack_depth, cudaStream_t stream) {
+    cudaError_t e = pool_alloc(t.device, &t.level_off, (size_t)(t.levels + 3) * sizeof(int32_t));
+    if (e != cudaSuccess) return e;
+    const Collapse C = collapse_view(t);
+    k_collapse_root<<<1, 1, 0, stream>>>(C);
+    for (int l = 0; l < t.levels; ++l) {
+        k_collapse_open<<<kCollapseGrid, 128, 0, stream>>>(bin_view(t), C, l, stack_depth);
+        k_collapse_level<<<1, 1, 0, stream>>>(C, l);
+    }
+    for (int l = t.levels - 1; l >= 0; --l) k_collapse_size<<<kCollapseGrid, 128, 0, stream>>>(bin_view(t), C, l);
+    e = cudaMemcpyAsync(&t.ncollapsed, C.tail, sizeof(int32_t), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    return e;
+}
+
+cudaError_t gpu_tree_emit(const GpuTree& t, void* d_nodes, int32_t* d_level_nodes, std::vector<int32_t>& level_off,
+                          cudaStream_t stream) {
+    const Collapse C = collapse_view(t);
+    for (int l = 0; l < t.levels; ++l)
+        k_collapse_emit<<<kCollapseGrid, 128, 0, stream>>>(bin_view(t), C, l, static_cast<GNode4*>(d_nodes), d_level_nodes);
+    level_off.resize((size_t)t.levels + 2);
+    cudaError_t e = cudaMemcpyAsync(level_off.data(), t.level_off, level_off.size() * sizeof(int32_t),
+                                    cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    // levels below the collapsed tree's depth are empty
+    while (level_off.size() > 2 && level_off[level_off.size() - 2] == level_off.back()) level_off.pop_back();
+    return e;
+}
+
+cudaError_t gpu_tree_download(const GpuTree& t, cudaStream_t stream, BinTree& out) {
+    out = BinTree();
+    const size_t m = (size_t)t.nnodes;
+    std::vector<float> nlo(3 * m), nhi(3 * m);
+    std::vector<int32_t> nl(m), nr(m), nf(m), nc(m), order((size_t)t.n);
+    cudaError_t e = cudaStreamSynchronize(stream);
+    auto get = [&](void* dst, const void* src, size_t bytes) {
+        if (e == cudaSuccess) e = cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
+    };
+    get(nlo.data(), t.lo, 12 * m);
+    get(nhi.data(), t.hi, 12 * m);
+    get(nl.data(), t.left, 4 * m);
+    get(nr.data(), t.right, 4 * m);
+    get(nf.data(), t.first, 4 * m);
+    get(nc.data(), t.count, 4 * m);
+    get(order.data(), t.order, 4 * (size_t)t.n);
+    if (e != cudaSuccess) return e;
     // pre-order renumbering (left subtree before right), as the host builder's flatten
-    out.nodes.reserve(nnodes);
+    out.nodes.reserve(m);
     struct Item {
         int32_t id, parent, depth;
         bool right;
@@ -617,7 +911,7 @@ bool build_sah_gpu(const std::vector<float>& tri_lo, const std::vector<float>& t
         }
     }
     out.order = std::move(order);
-    return true;
+    return cudaSuccess;
 }
 
 }  // namespace sbr

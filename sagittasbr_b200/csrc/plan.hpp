@@ -24,10 +24,7 @@ struct sbr_scene {
     int64_t ntris = 0;
     double model_scale = 1.0;
     double aabb_lo[3] = {0, 0, 0}, aabb_hi[3] = {0, 0, 0};  // conservative, FP64
-    // host copies kept for the FP64 upload and diagnostics
-    std::vector<float> xyz;          // caller vertices (unscaled)
-    std::vector<uint32_t> idx;
-    std::vector<int32_t> order;      // leaf slot -> caller triangle index
+    int64_t nverts = 0;
     // device: one block (nodes to d_cancel), the others apart
     void* block = nullptr;
     sbr::GNode4* d_nodes = nullptr;
@@ -42,7 +39,7 @@ struct sbr_scene {
     unsigned long long* d_horizon = nullptr;  // per slot: escape elevations by octant (horizon.cu)
     bool horizon_built = false;      // false after a refit: all bytes 255, every ray walks
     std::mutex horizon_mu;
-    float* d_xyz = nullptr;          // caller vertices and triangles, uploaded for the adjoint
+    float* d_xyz = nullptr;          // caller vertices (unscaled) and triangles
     uint32_t* d_idx = nullptr;
     uint32_t* d_err = nullptr;
     int32_t* d_cancel = nullptr;     // device word polled by the kernels
@@ -52,9 +49,8 @@ struct sbr_scene {
     int depth = 0;
     double build_ms = 0.0;
     double sah_ms = 0.0;
-    // refit: 4-wide node indices grouped by depth (offsets per depth), their device
-    // copy, and the per-triangle box scratch of a refit
-    std::vector<int32_t> refit_nodes;
+    // refit: 4-wide node indices grouped by depth (offsets per depth), and the
+    // per-triangle box scratch of a refit
     std::vector<int32_t> refit_level_off;
     int32_t* d_refit_nodes = nullptr;
     float* d_tri_box = nullptr;
@@ -179,7 +175,9 @@ sbr_status trace_list_launch(sbr_plan* pl, const int32_t* d_rays, long long n, s
 int max_freqs_per_job();
 int max_lane_channels();  // channels up to which every lane sums its own rays' terms
 sbr_status ensure_fp64(sbr_scene* s);
-sbr_status ensure_adjoint_data(sbr_scene* s);
+// Triangle records, their FP64 twins and boxes (any may be null) from the scene's
+// vertices, on its stream.
+sbr_status write_triangles(sbr_scene* s, GTri* tris, GTri64* tris64, float* box);
 // Computes the scene's horizons unless it holds them, and waits for them.
 sbr_status build_horizons(sbr_scene* s);
 // Takes them back, in stream order, so that every ray walks (plans that exist see it).

@@ -6,8 +6,9 @@
 // vertices a little.
 //
 //   k_refit_tris   one thread per leaf slot: the triangle's FP32 data (v0, v1, v2,
-//                  unit normal) in exactly the host set-up's arithmetic (scene.cpp:
-//                  products and sums rounded one by one, no contraction), its FP64
+//                  unit normal; the scene's set-up writes them with the same kernel), in
+//                  the reference's FP32 arithmetic (src/cuda/rtKernels.cu:13-14,42; products
+//                  and sums rounded one by one, no contraction), its FP64
 //                  twin when the scene has one, and its conservative box (covering
 //                  the FP32 and the outward-rounded FP64 vertices);
 //   k_refit_level  one thread per 4-wide node of one depth, deepest depth first:
@@ -43,10 +44,11 @@ __global__ void k_refit_tris(const float* __restrict__ xyz, const uint32_t* __re
             hi[a] = fmaxf(hi[a], fmaxf(p[c][a], __double2float_ru(q[c][a])));
         }
     }
-    for (int a = 0; a < 3; ++a) {
-        box[6 * slot + a] = lo[a];
-        box[6 * slot + 3 + a] = hi[a];
-    }
+    if (box)
+        for (int a = 0; a < 3; ++a) {
+            box[6 * slot + a] = lo[a];
+            box[6 * slot + 3 + a] = hi[a];
+        }
     float e1[3], e2[3];
     for (int a = 0; a < 3; ++a) {
         e1[a] = __fsub_rn(p[1][a], p[0][a]);
@@ -66,7 +68,7 @@ __global__ void k_refit_tris(const float* __restrict__ xyz, const uint32_t* __re
     g.v0 = make_float4(p[0][0], p[0][1], p[0][2], n[0]);
     g.v1 = make_float4(p[1][0], p[1][1], p[1][2], n[1]);
     g.v2 = make_float4(p[2][0], p[2][1], p[2][2], n[2]);
-    tris[slot] = g;
+    if (tris) tris[slot] = g;
     if (tris64) {
         GTri64 h;
         for (int a = 0; a < 3; ++a) {
@@ -126,40 +128,41 @@ __global__ void k_refit_level(GNode4* nodes, const int32_t* __restrict__ level_n
 }
 
 }  // namespace
+
+sbr_status write_triangles(sbr_scene* s, GTri* tris, GTri64* tris64, float* box) {
+    const unsigned gt = (unsigned)((s->ntris + kRefitThreads - 1) / kRefitThreads);
+    k_refit_tris<<<gt, kRefitThreads, 0, s->stream>>>(s->d_xyz, s->d_idx, s->d_tri_id, s->ntris, float(s->model_scale),
+                                                      s->model_scale, tris, tris64, box);
+    SBR_CUDA(cudaGetLastError());
+    return SBR_OK;
+}
+
 }  // namespace sbr
 
 extern "C" sbr_status sbr_scene_update_vertices(sbr_scene* s, const float* xyz, size_t nverts) {
     using namespace sbr;
     if (!s || !xyz) return fail(SBR_ERR_INVALID_ARG, "scene and vertices are required");
-    if (nverts * 3 != s->xyz.size()) return fail(SBR_ERR_INVALID_ARG, "vertex count differs from the scene's");
+    if ((int64_t)nverts != s->nverts) return fail(SBR_ERR_INVALID_ARG, "vertex count differs from the scene's");
     for (size_t i = 0; i < 3 * nverts; ++i)
         if (!std::isfinite(xyz[i])) return fail(SBR_ERR_NONFINITE, "non-finite vertex coordinate");
     sbr::DeviceGuard device_guard;
     SBR_CUDA(cudaSetDevice(s->device));
-    sbr_status st = ensure_adjoint_data(s);  // device copies of the caller's vertices and triangles
-    if (st != SBR_OK) return st;
+    sbr_status st;
     if (s->d_nodes8) {  // the opt-in 8-wide tree is not refitted: the sweep walks the 4-wide one again
         SBR_CUDA(cudaDeviceSynchronize());  // plans on other streams may still walk it
         pool_free(s->device, s->d_nodes8);
         s->d_nodes8 = nullptr;
         s->n_gnodes8 = 0;
     }
-    if (!s->d_refit_nodes) {
-        const size_t nb = s->refit_nodes.size() * sizeof(int32_t), bb = 6 * (size_t)s->ntris * sizeof(float);
-        if (pool_alloc(s->device, &s->d_refit_nodes, nb) != cudaSuccess ||
-            pool_alloc(s->device, &s->d_tri_box, bb) != cudaSuccess)
-            return fail(SBR_ERR_OOM, "refit buffers");
-        SBR_CUDA(cudaMemcpy(s->d_refit_nodes, s->refit_nodes.data(), nb, cudaMemcpyHostToDevice));
-        s->device_bytes += (int64_t)(nb + bb);
+    if (!s->d_tri_box) {
+        const size_t bb = 6 * (size_t)s->ntris * sizeof(float);
+        if (pool_alloc(s->device, &s->d_tri_box, bb) != cudaSuccess) return fail(SBR_ERR_OOM, "refit buffers");
+        s->device_bytes += (int64_t)bb;
     }
-    s->xyz.assign(xyz, xyz + 3 * nverts);
     if ((st = clear_horizons(s)) != SBR_OK) return st;
     cudaStream_t st_ = s->stream;
-    SBR_CUDA(cudaMemcpyAsync(s->d_xyz, s->xyz.data(), s->xyz.size() * sizeof(float), cudaMemcpyHostToDevice, st_));
-    const unsigned gt = (unsigned)((s->ntris + kRefitThreads - 1) / kRefitThreads);
-    k_refit_tris<<<gt, kRefitThreads, 0, st_>>>(s->d_xyz, s->d_idx, s->d_tri_id, s->ntris, float(s->model_scale),
-                                                 s->model_scale, s->d_tris, s->d_tris64, s->d_tri_box);
-    SBR_CUDA(cudaGetLastError());
+    SBR_CUDA(cudaMemcpyAsync(s->d_xyz, xyz, 3 * nverts * sizeof(float), cudaMemcpyHostToDevice, st_));
+    if ((st = write_triangles(s, s->d_tris, s->d_tris64, s->d_tri_box)) != SBR_OK) return st;
     const std::vector<int32_t>& off = s->refit_level_off;
     for (size_t d = off.size() - 1; d-- > 0;) {
         const int32_t n = off[d + 1] - off[d];

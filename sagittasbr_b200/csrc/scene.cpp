@@ -64,8 +64,7 @@ void free_scene(sbr_scene* s) {
     cudaGetDevice(&cur);
     cudaSetDevice(s->device);
     cudaDeviceSynchronize();  // plans on the caller's streams may still walk the scene
-    for (void* q : {s->block, (void*)s->d_nodes8, (void*)s->d_tris64, (void*)s->d_xyz, (void*)s->d_idx,
-                    (void*)s->d_refit_nodes, (void*)s->d_tri_box})
+    for (void* q : {s->block, (void*)s->d_nodes8, (void*)s->d_tris64, (void*)s->d_xyz, (void*)s->d_tri_box})
         pool_free(s->device, q);
     pool_close(s->device);
     if (s->cancel_stream) cudaStreamDestroy(s->cancel_stream);
@@ -82,28 +81,21 @@ namespace sbr {
 
 sbr_status ensure_fp64(sbr_scene* s) {
     if (s->d_tris64) return SBR_OK;
-    std::vector<GTri64> t64(s->ntris);
-    for (int64_t slot = 0; slot < s->ntris; ++slot) {
-        int32_t t = s->order[slot];
-        double a[3], b[3], c[3];
-        vert64(s->xyz.data(), s->idx[3 * t], s->model_scale, a);
-        vert64(s->xyz.data(), s->idx[3 * t + 1], s->model_scale, b);
-        vert64(s->xyz.data(), s->idx[3 * t + 2], s->model_scale, c);
-        GTri64& g = t64[slot];
-        for (int k = 0; k < 3; ++k) { g.v0[k] = a[k]; g.e1[k] = b[k] - a[k]; g.e2[k] = c[k] - a[k]; }
-        double nx = g.e1[1] * g.e2[2] - g.e1[2] * g.e2[1];
-        double ny = -(g.e1[0] * g.e2[2] - g.e1[2] * g.e2[0]);
-        double nz = g.e1[0] * g.e2[1] - g.e1[1] * g.e2[0];
-        double len = std::sqrt(nx * nx + ny * ny + nz * nz);
-        if (len > 0) { g.n[0] = nx / len; g.n[1] = ny / len; g.n[2] = nz / len; }
-        else { g.n[0] = g.n[1] = g.n[2] = 0.0; }
-    }
     sbr::DeviceGuard device_guard;
     SBR_CUDA(cudaSetDevice(s->device));
-    size_t bytes = sizeof(GTri64) * t64.size();
-    cudaError_t e = pool_alloc(s->device, &s->d_tris64, bytes);
-    if (e != cudaSuccess) return fail(SBR_ERR_OOM, "allocation of FP64 triangles failed");
-    SBR_CUDA(cudaMemcpy(s->d_tris64, t64.data(), bytes, cudaMemcpyHostToDevice));
+    const size_t bytes = sizeof(GTri64) * (size_t)s->ntris;
+    GTri64* t64 = nullptr;
+    if (pool_alloc(s->device, &t64, bytes) != cudaSuccess)
+        return fail(SBR_ERR_OOM, "allocation of FP64 triangles failed");
+    // plans may launch on the caller's streams: the triangles are there when this returns
+    sbr_status st = write_triangles(s, nullptr, t64, nullptr);
+    const cudaError_t e = cudaStreamSynchronize(s->stream);
+    if (st == SBR_OK && e != cudaSuccess) st = cuda_fail(e, "FP64 triangles");
+    if (st != SBR_OK) {
+        pool_free(s->device, t64);
+        return st;
+    }
+    s->d_tris64 = t64;
     s->device_bytes += (int64_t)bytes;
     return SBR_OK;
 }
@@ -149,27 +141,43 @@ sbr_status sbr_scene_create(const float* xyz, size_t nverts, const uint32_t* tri
     s->num_sms = num_sms;
     s->ntris = (int64_t)ntris;
     s->model_scale = scale;
-    s->xyz.assign(xyz, xyz + 3 * nverts);
-    s->idx.assign(tri_idx, tri_idx + 3 * ntris);
+    s->nverts = (int64_t)nverts;
 
-    // per-triangle conservative boxes (cover both the FP32 and FP64 vertices)
-    const float sc32 = float(scale);
-    std::vector<float> lo(3 * ntris), hi(3 * ntris);
-    parallel_for(ntris, o.n_threads, [&](size_t t0, size_t t1) {
-        for (size_t t = t0; t < t1; ++t) {
-            for (int a = 0; a < 3; ++a) { lo[3 * t + a] = INFINITY; hi[3 * t + a] = -INFINITY; }
-            for (int c = 0; c < 3; ++c) {
-                float p32[3];
-                double p64[3];
-                vert32(xyz, tri_idx[3 * t + c], sc32, p32);
-                vert64(xyz, tri_idx[3 * t + c], scale, p64);
-                for (int a = 0; a < 3; ++a) {
-                    lo[3 * t + a] = std::min({lo[3 * t + a], p32[a], round_down(p64[a])});
-                    hi[3 * t + a] = std::max({hi[3 * t + a], p32[a], round_up(p64[a])});
-                }
-            }
-        }
-    });
+    GpuTree gt;
+    int32_t* twins = nullptr;  // hash table of the search for coincident faces, and its answer
+    auto bail = [&](sbr_status st) {
+        if (s->stream) gpu_tree_free(gt, s->stream);
+        cudaDeviceSynchronize();
+        pool_free(dev, twins);
+        free_scene(s);
+        return st;
+    };
+    cudaError_t e;
+    if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaStreamCreateWithFlags(&s->cancel_stream, cudaStreamNonBlocking)) != cudaSuccess)
+        return bail(cuda_fail(e, "cudaStreamCreate"));
+    auto no_memory = [&]() {
+        return bail(fail(SBR_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(e)));
+    };
+    // the caller's mesh, from which the kernels make the triangle records (and the tree)
+    {
+        Parts parts;
+        const size_t vb = 3 * nverts * sizeof(float), ib = 3 * ntris * sizeof(uint32_t);
+        const size_t v_at = parts.add(vb), i_at = parts.add(ib);
+        char* m = nullptr;
+        if ((e = pool_alloc(dev, &m, parts.size())) != cudaSuccess) return no_memory();
+        s->d_xyz = reinterpret_cast<float*>(m + v_at);
+        s->d_idx = reinterpret_cast<uint32_t*>(m + i_at);
+        s->device_bytes += (int64_t)parts.size();
+        if ((e = cudaMemcpyAsync(s->d_xyz, xyz, vb, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess ||
+            (e = cudaMemcpyAsync(s->d_idx, tri_idx, ib, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess)
+            return bail(cuda_fail(e, "mesh upload"));
+    }
+    const size_t table = gpu_twins_table(ntris);
+    if ((e = pool_alloc(dev, &twins, (table + 1) * sizeof(int32_t))) != cudaSuccess) return no_memory();
+    if ((e = gpu_opposed_twins(s->d_xyz, s->d_idx, ntris, twins, twins + table, s->stream)) != cudaSuccess)
+        return bail(cuda_fail(e, "coincident faces"));
+
     BuildOptions bo;
     // 3, not the reference's 4 (src/scene/bvhBuilder.hpp:14): with 4-wide nodes one
     // more level of boxes is cheaper than a fourth triangle test per leaf (trihedral
@@ -180,23 +188,49 @@ sbr_status sbr_scene_create(const float* xyz, size_t nverts, const uint32_t* tri
     bo.max_leaf = kLeafMax;
     const auto ts0 = std::chrono::steady_clock::now();
     BinTree tree;
-    if (o.gpu_build > 0) {
-        cudaStream_t bs = nullptr;
-        cudaError_t be = cudaStreamCreateWithFlags(&bs, cudaStreamNonBlocking);
-        const bool ok = be == cudaSuccess && build_sah_gpu(lo, hi, bo, bs, tree, &be);
-        if (bs) cudaStreamDestroy(bs);
-        if (!ok) {
-            free_scene(s);
-            return cuda_fail(be, "GPU BVH build");
-        }
+    const bool on_gpu = o.gpu_build > 0;
+    // (the 8-wide tree is made from a tree on the host)
+    const bool collapse_on_gpu = on_gpu && o.node_width != 8;
+    if (on_gpu) {
+        e = gpu_tree_build(s->d_xyz, s->d_idx, (int)ntris, scale, bo, s->stream, gt);
+        if (e == cudaSuccess && !collapse_on_gpu) e = gpu_tree_download(gt, s->stream, tree);
+        if (e != cudaSuccess) return bail(cuda_fail(e, "GPU BVH build"));
     } else {
+        // per-triangle conservative boxes (cover both the FP32 and FP64 vertices)
+        const float sc32 = float(scale);
+        std::vector<float> lo(3 * ntris), hi(3 * ntris);
+        parallel_for(ntris, o.n_threads, [&](size_t t0, size_t t1) {
+            for (size_t t = t0; t < t1; ++t) {
+                for (int a = 0; a < 3; ++a) { lo[3 * t + a] = INFINITY; hi[3 * t + a] = -INFINITY; }
+                for (int c = 0; c < 3; ++c) {
+                    float p32[3];
+                    double p64[3];
+                    vert32(xyz, tri_idx[3 * t + c], sc32, p32);
+                    vert64(xyz, tri_idx[3 * t + c], scale, p64);
+                    for (int a = 0; a < 3; ++a) {
+                        lo[3 * t + a] = std::min({lo[3 * t + a], p32[a], round_down(p64[a])});
+                        hi[3 * t + a] = std::max({hi[3 * t + a], p32[a], round_up(p64[a])});
+                    }
+                }
+            }
+        });
         tree = build_sah(lo, hi, bo);
     }
     s->sah_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - ts0).count();
-    s->order = tree.order;
-    s->n_bin_nodes = (int64_t)tree.nodes.size();
-    s->depth = tree.depth;
-    for (int a = 0; a < 3; ++a) { s->aabb_lo[a] = tree.nodes[0].lo[a]; s->aabb_hi[a] = tree.nodes[0].hi[a]; }
+    if (collapse_on_gpu) {
+        float box[6];
+        e = cudaMemcpyAsync(box, gt.lo, 3 * sizeof(float), cudaMemcpyDeviceToHost, s->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(box + 3, gt.hi, 3 * sizeof(float), cudaMemcpyDeviceToHost, s->stream);
+        if (e == cudaSuccess) e = gpu_tree_collapse(gt, kStackDepth, s->stream);
+        if (e != cudaSuccess) return bail(cuda_fail(e, "GPU BVH collapse"));
+        s->n_bin_nodes = gt.nnodes;
+        s->depth = gt.levels;
+        for (int a = 0; a < 3; ++a) { s->aabb_lo[a] = box[a]; s->aabb_hi[a] = box[3 + a]; }
+    } else {
+        s->n_bin_nodes = (int64_t)tree.nodes.size();
+        s->depth = tree.depth;
+        for (int a = 0; a < 3; ++a) { s->aabb_lo[a] = tree.nodes[0].lo[a]; s->aabb_hi[a] = tree.nodes[0].hi[a]; }
+    }
 
     // GPU nodes: the binary tree collapsed to 4-wide nodes.  A 4-wide node takes a
     // binary node's two children and keeps opening its largest (by surface area)
@@ -218,7 +252,9 @@ sbr_status sbr_scene_create(const float* xyz, size_t nverts, const uint32_t* tri
         (&n.loz.x)[c] = lo[2]; (&n.hiz.x)[c] = hi[2];
         (&n.child.x)[c] = ref;
     };
-    if (tree.nodes[0].left < 0) {
+    if (collapse_on_gpu) {
+        // (written below, once the device block is there)
+    } else if (tree.nodes[0].left < 0) {
         GNode4 n;
         fill(n, 0, &tree.nodes[0], leafRef(tree.nodes[0]));
         for (int c = 1; c < 4; ++c) fill(n, c, nullptr, ~0);
@@ -277,7 +313,7 @@ sbr_status sbr_scene_create(const float* xyz, size_t nverts, const uint32_t* tri
             for (int q = ni - 1; q >= 0; --q) work.push_back(inner[q]);
         }
     }
-    s->n_gnodes = (int64_t)g.size();
+    s->n_gnodes = collapse_on_gpu ? gt.ncollapsed : (int64_t)g.size();
 
     // Opt-in 8-wide tree over the same leaves: the same greedy collapse, opening
     // the largest inner child until a node holds eight children (or the walker's
@@ -339,91 +375,78 @@ sbr_status sbr_scene_create(const float* xyz, size_t nverts, const uint32_t* tri
     }
     s->n_gnodes8 = (int64_t)g8.size();
     // nodes grouped by depth (a refit recomputes the boxes deepest level first)
-    {
+    std::vector<int32_t> level_nodes;
+    if (!collapse_on_gpu) {
         const int32_t maxd = *std::max_element(level.begin(), level.end());
         s->refit_level_off.assign((size_t)maxd + 2, 0);
         for (int32_t d : level) ++s->refit_level_off[(size_t)d + 1];
         for (size_t d = 1; d < s->refit_level_off.size(); ++d) s->refit_level_off[d] += s->refit_level_off[d - 1];
         std::vector<int32_t> fillp(s->refit_level_off.begin(), s->refit_level_off.end() - 1);
-        s->refit_nodes.resize(g.size());
-        for (size_t k = 0; k < g.size(); ++k) s->refit_nodes[(size_t)fillp[(size_t)level[k]]++] = (int32_t)k;
+        level_nodes.resize(g.size());
+        for (size_t k = 0; k < g.size(); ++k) level_nodes[(size_t)fillp[(size_t)level[k]]++] = (int32_t)k;
     }
 
-    // leaf-ordered triangles: v0, v1, v2 in FP32 and the unit normal unit(e1 x e2)
-    // with e1, e2 in the reference's FP32 arithmetic (src/cuda/rtKernels.cu:13-14,42)
-    std::vector<GTri> tr(ntris);
-    std::vector<int32_t> ids(ntris);
-    parallel_for(ntris, o.n_threads, [&](size_t s0, size_t s1) {
-        for (size_t slot = s0; slot < s1; ++slot) {
-            int32_t t = s->order[slot];
-            ids[slot] = t;
-            float a[3], b[3], c[3];
-            vert32(xyz, tri_idx[3 * t], sc32, a);
-            vert32(xyz, tri_idx[3 * t + 1], sc32, b);
-            vert32(xyz, tri_idx[3 * t + 2], sc32, c);
-            float e1[3] = {b[0] - a[0], b[1] - a[1], b[2] - a[2]};
-            float e2[3] = {c[0] - a[0], c[1] - a[1], c[2] - a[2]};
-            float nx = e1[1] * e2[2] - e1[2] * e2[1];
-            float ny = -(e1[0] * e2[2] - e1[2] * e2[0]);
-            float nz = e1[0] * e2[1] - e1[1] * e2[0];
-            float len = std::sqrt(nx * nx + ny * ny + nz * nz);
-            float n[3] = {0.0f, 0.0f, 0.0f};
-            if (len > 0.0f) { n[0] = nx / len; n[1] = ny / len; n[2] = nz / len; }
-            tr[slot].v0 = make_float4(a[0], a[1], a[2], n[0]);
-            tr[slot].v1 = make_float4(b[0], b[1], b[2], n[1]);
-            tr[slot].v2 = make_float4(c[0], c[1], c[2], n[2]);
-        }
-    });
     // exact ties: where the mesh holds a triangle twice with opposite windings, each
     // slot's rank in the reference's walk order decides which of two equally near
     // triangles a ray keeps (the reference keeps the last it tests)
     std::vector<int32_t> tie;
-    if (has_opposed_twins(xyz, tri_idx, ntris)) {
+    int32_t has_twins = 0;
+    if ((e = cudaMemcpyAsync(&has_twins, twins + table, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s->stream)) != cudaSuccess)
+        return bail(cuda_fail(e, "coincident faces"));
+    pool_free(dev, twins);
+    twins = nullptr;
+    if (has_twins) {
+        if (collapse_on_gpu) {
+            tree.order.resize(ntris);
+            if ((e = cudaMemcpy(tree.order.data(), gt.order, sizeof(int32_t) * ntris, cudaMemcpyDeviceToHost)) != cudaSuccess)
+                return bail(cuda_fail(e, "triangle order"));
+        }
         const std::vector<int32_t> rank = reference_walk_rank(xyz, tri_idx, ntris, scale, o.n_threads);
         tie.resize(ntris);
-        for (size_t slot = 0; slot < ntris; ++slot) tie[slot] = rank[(size_t)s->order[slot]];
+        for (size_t slot = 0; slot < ntris; ++slot) tie[slot] = rank[(size_t)tree.order[slot]];
     }
     auto t1 = std::chrono::steady_clock::now();
     s->build_ms = std::chrono::duration<double, std::milli>(t1 - t0).count();
 
-    auto bail = [&](sbr_status st) {
-        free_scene(s);
-        return st;
-    };
-    cudaError_t e;
-    const size_t nb = sizeof(GNode4) * g.size(), tb = sizeof(GTri) * tr.size(), ib = sizeof(int32_t) * ids.size(),
-                 hb = sizeof(unsigned long long) * ntris, rb = sizeof(int32_t) * tie.size();
+    const size_t nb = sizeof(GNode4) * (size_t)s->n_gnodes, tb = sizeof(GTri) * ntris, ib = sizeof(int32_t) * ntris,
+                 hb = sizeof(unsigned long long) * ntris, lb = sizeof(int32_t) * (size_t)s->n_gnodes,
+                 rb = sizeof(int32_t) * tie.size();
     Parts parts;
     const size_t node_at = parts.add(nb), tri_at = parts.add(tb), id_at = parts.add(ib), hor_at = parts.add(hb),
-                 tie_at = parts.add(rb), err_at = parts.add(sizeof(uint32_t)), cancel_at = parts.add(sizeof(int32_t));
+                 level_at = parts.add(lb), tie_at = parts.add(rb), err_at = parts.add(sizeof(uint32_t)), cancel_at = parts.add(sizeof(int32_t));
     char* b = nullptr;
-    if ((e = pool_alloc(dev, &b, parts.size())) != cudaSuccess)
-        return bail(fail(SBR_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(e)));
+    if ((e = pool_alloc(dev, &b, parts.size())) != cudaSuccess) return no_memory();
     s->block = b;
     s->d_nodes = reinterpret_cast<GNode4*>(b + node_at);
     s->d_tris = reinterpret_cast<GTri*>(b + tri_at);
     s->d_tri_id = reinterpret_cast<int32_t*>(b + id_at);
     s->d_horizon = reinterpret_cast<unsigned long long*>(b + hor_at);
+    s->d_refit_nodes = reinterpret_cast<int32_t*>(b + level_at);
     if (rb) s->d_tie = reinterpret_cast<int32_t*>(b + tie_at);
     s->d_err = reinterpret_cast<uint32_t*>(b + err_at);
     // cancel flag: a device word (the kernels poll it from L2); the host sets it on a side
     // stream, which runs while the sweep kernel is resident
     s->d_cancel = reinterpret_cast<int32_t*>(b + cancel_at);
-    if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess ||
-        (e = cudaStreamCreateWithFlags(&s->cancel_stream, cudaStreamNonBlocking)) != cudaSuccess)
-        return bail(cuda_fail(e, "cudaStreamCreate"));
-    if ((e = cudaMemcpyAsync(s->d_nodes, g.data(), nb, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(s->d_tris, tr.data(), tb, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(s->d_tri_id, ids.data(), ib, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess ||
+    if (collapse_on_gpu) {
+        e = cudaMemcpyAsync(s->d_tri_id, gt.order, ib, cudaMemcpyDeviceToDevice, s->stream);
+        if (e == cudaSuccess) e = gpu_tree_emit(gt, s->d_nodes, s->d_refit_nodes, s->refit_level_off, s->stream);
+    } else {
+        e = cudaMemcpyAsync(s->d_nodes, g.data(), nb, cudaMemcpyHostToDevice, s->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(s->d_tri_id, tree.order.data(), ib, cudaMemcpyHostToDevice, s->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(s->d_refit_nodes, level_nodes.data(), lb, cudaMemcpyHostToDevice, s->stream);
+    }
+    if (e != cudaSuccess ||
         (rb && (e = cudaMemcpyAsync(s->d_tie, tie.data(), rb, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess) ||
         (e = cudaMemsetAsync(s->d_err, 0, sizeof(uint32_t), s->stream)) != cudaSuccess ||
         (e = cudaMemsetAsync(s->d_cancel, 0, sizeof(int32_t), s->stream)) != cudaSuccess)
         return bail(cuda_fail(e, "scene upload"));
-    s->device_bytes = (int64_t)parts.size();
+    s->device_bytes += (int64_t)parts.size();
+    sbr_status ws = write_triangles(s, s->d_tris, nullptr, nullptr);
+    if (ws != SBR_OK) return bail(ws);
     if (!g8.empty()) {
         const size_t nb8 = sizeof(GNode8) * g8.size();
-        if ((e = pool_alloc(dev, &s->d_nodes8, nb8)) != cudaSuccess)
-            return bail(fail(SBR_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(e)));
+        if ((e = pool_alloc(dev, &s->d_nodes8, nb8)) != cudaSuccess) return no_memory();
         if ((e = cudaMemcpyAsync(s->d_nodes8, g8.data(), nb8, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess)
             return bail(cuda_fail(e, "8-wide node upload"));
         s->device_bytes += (int64_t)nb8;
@@ -431,6 +454,7 @@ sbr_status sbr_scene_create(const float* xyz, size_t nverts, const uint32_t* tri
     // (waits for the uploads as well)
     sbr_status hs = build_horizons(s);
     if (hs != SBR_OK) return bail(hs);
+    gpu_tree_free(gt, s->stream);
     if (o.want_fp64 > 0) {
         sbr_status st = ensure_fp64(s);
         if (st != SBR_OK) return bail(st);
