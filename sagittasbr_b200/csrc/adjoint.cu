@@ -296,6 +296,7 @@ extern "C" sbr_status sbr_adjoint(sbr_scene* s, const sbr_job* jobs, size_t n_jo
     if (ns) SBR_CUDA(cudaMemcpyAsync(d_cot, cot, 2 * ns * sizeof(double), cudaMemcpyHostToDevice, stream));
     SBR_CUDA(cudaMemsetAsync(B.block, 0, zero_b, stream));
 
+    if ((st = plan_horizons(p)) != SBR_OK) return st;
     if (p->n_items > 0) {
         const void* fn = pick_adjoint(p->prec);
         int occ = 0;

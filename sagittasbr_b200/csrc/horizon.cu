@@ -30,13 +30,24 @@
 // horizon.  The FP32 mode's Moller-Trumbore test can report hits well outside a
 // triangle near grazing incidence, so that mode does not use horizons.
 //
+// A scene starts without horizons (all bytes 255: every ray walks) and gets them, in the
+// stream of the sweep that needs them, once its sweeps have launched kHorizonRays rays per
+// triangle.  They cost 5 to 15 ns a triangle and save 2 to 130 ps a launched ray (break-even
+// at 60 rays per triangle on a smooth ellipsoid, 120 on a small sphere, 650 on a coarse
+// aircraft, 3,900 on a fine jittered one seen from the nose), and a ray costs 30 to 100 ps:
+// at 1,500 the sweep that brings them is at most a tenth longer for it, and a first look at
+// a new model, or a step that moves the vertices again, does not pay for what it cannot
+// use (at 200 a first sweep took up to 36 % longer).
+// The bytes change in place: a plan or graph made before reads them too, and a kernel that
+// runs meanwhile sees 255 or the final byte.
+//
 // The search walks the 4-wide tree once per triangle, children with the largest bound
 // first, and drops a box when its bound A is below the octants' current H or below
 // kFloor; a box seen under less than kAccept is taken by its bound instead of being
 // opened.  One thread per slot: neighbouring slots are neighbouring triangles, so a
 // warp's walks stay together (mean visits 126, mean of a warp's longest 198 on the
-// aircraft).  Bound by the bounds' arithmetic, 9.8 ns a triangle there (21 ms of about
-// 0.4 s of scene set-up; 0.3 ms for a 20k-triangle sphere).  Measured on the aircraft's
+// aircraft).  Bound by the bounds' arithmetic, 9.8 ns a triangle there (21 ms;
+// 0.3 ms for a 20k-triangle sphere).  Measured on the aircraft's
 // 10 azimuths from the nose, floor / accept: 0.1 / 0.12 35.9 ms and 52.6 M of the 80.6 M
 // second queries still walked, 0.1 / 0.25 22.2 ms and 53.2 M, 0.15 / 0.25 21.0 ms and
 // 54.1 M, 0.2 / 0.25 19.7 ms and 55.5 M; broadside 30 % still walk.
@@ -55,6 +66,7 @@ namespace {
 constexpr float kFloor = 0.15f;      // smallest horizon told apart
 constexpr unsigned kTop = 229;       // byte (0.9) from which a direction counts as blocked
 constexpr float kAccept = 0.25f;     // diagonal / (2 distance) below which a box is not opened
+constexpr int64_t kHorizonRays = 1500; // launched rays per triangle from which a scene has them
 constexpr int kVisits = 4096;        // node visits per triangle before it is given up (blocked)
 constexpr float kU32 = 5.9604644775390625e-08f;  // 2^-24
 
@@ -265,21 +277,28 @@ __global__ void __launch_bounds__(128) k_horizon(const GNode4* __restrict__ node
 
 }  // namespace
 
-sbr_status build_horizons(sbr_scene* s) {
+sbr_status use_horizons(sbr_scene* s, int64_t rays, cudaStream_t stream) {
     std::lock_guard<std::mutex> lock(s->horizon_mu);
     if (s->horizon_built) return SBR_OK;
-    k_horizon<<<(unsigned)((s->ntris + 127) / 128), 128, 0, s->stream>>>(s->d_nodes, s->d_tris, s->ntris, s->d_horizon);
+    s->horizon_rays += rays;
+    if (s->horizon_rays < kHorizonRays * s->ntris) return SBR_OK;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    SBR_CUDA(cudaStreamIsCapturing(stream, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return SBR_OK;  // not into somebody's graph
+    if (!s->horizon_done) SBR_CUDA(cudaEventCreateWithFlags(&s->horizon_done, cudaEventDisableTiming));
+    k_horizon<<<(unsigned)((s->ntris + 127) / 128), 128, 0, stream>>>(s->d_nodes, s->d_tris, s->ntris, s->d_horizon);
     SBR_CUDA(cudaGetLastError());
-    // plans may launch on the caller's streams, which the scene's does not hold up
-    SBR_CUDA(cudaStreamSynchronize(s->stream));
+    SBR_CUDA(cudaEventRecord(s->horizon_done, stream));
     s->horizon_built = true;
     return SBR_OK;
 }
 
 sbr_status clear_horizons(sbr_scene* s) {
     std::lock_guard<std::mutex> lock(s->horizon_mu);
+    if (s->horizon_done) SBR_CUDA(cudaStreamWaitEvent(s->stream, s->horizon_done, 0));
     SBR_CUDA(cudaMemsetAsync(s->d_horizon, 0xff, sizeof(unsigned long long) * (size_t)s->ntris, s->stream));
     s->horizon_built = false;
+    s->horizon_rays = 0;
     return SBR_OK;
 }
 

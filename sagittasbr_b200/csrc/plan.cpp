@@ -92,6 +92,14 @@ sbr_status check_device_errors(sbr_plan* p) {
 
 namespace sbr {
 
+sbr_status plan_horizons(sbr_plan* p) {
+    for (const auto& r : p->scene_rays) {
+        sbr_status st = use_horizons(r.first, r.second, p->stream);
+        if (st != SBR_OK) return st;
+    }
+    return SBR_OK;
+}
+
 sbr_status plan_fork(sbr_plan* p) {
     sbr_scene* s = p->scene;
     if (!p->side) {
@@ -494,14 +502,10 @@ sbr_status plan_create(sbr_scene* const* scenes, size_t n_scenes, const int32_t*
     p->n_pol = p->pol == SBR_POL_HHVV ? 2 : 1;
     if (o.mode == SBR_MODE_BATCHED && o.blocks_per_item == 0)
         cut_items(p, o.precision == SBR_PREC_MIXED && p->k_max * p->n_pol > max_lane_channels());
-    // a refitted scene has no horizons: a plan that launches enough rays to pay for them
-    // (5 to 20 ns a triangle against 50 to 100 ps a ray, measured on B200) brings them back
-    if (!p->multi && p->prec != SBR_PREC_FP32 && p->n_rays_clipped >= 200 * s->ntris) {
-        sbr_status st = build_horizons(s);
-        if (st != SBR_OK) {
-            release(p);
-            return st;
-        }
+    if (p->prec != SBR_PREC_FP32) {
+        for (size_t k = 0; k < (p->multi ? n_scenes : 1); ++k) p->scene_rays.emplace_back(scenes[k], 0);
+        for (const Segment& g : p->segs)
+            p->scene_rays[p->multi ? (size_t)p->jobs[g.job].scene : 0].second += (int64_t)g.ni * g.nj;
     }
     if (p->n_pol == 2) {
         // per angle: HH / VV unit vectors and the reference launch plane; the
@@ -674,6 +678,8 @@ sbr_status sbr_plan_execute(sbr_plan* p) {
     sbr::DeviceGuard device_guard;
     SBR_CUDA(cudaSetDevice(p->device));
     SBR_CUDA(cudaEventRecord(p->ev0, p->stream));
+    sbr_status hs = plan_horizons(p);
+    if (hs != SBR_OK) return hs;
     if (p->use_graph && p->mode == SBR_MODE_BATCHED) {
         if (!p->graph) {
             // size the persistent grid outside capture, then capture the launches

@@ -37,7 +37,9 @@ struct sbr_scene {
     int32_t* d_tri_id = nullptr;
     int32_t* d_tie = nullptr;        // exact-tie ranks (coincident faces of opposite winding), or null
     unsigned long long* d_horizon = nullptr;  // per slot: escape elevations by octant (horizon.cu)
-    bool horizon_built = false;      // false after a refit: all bytes 255, every ray walks
+    bool horizon_built = false;      // false: all bytes 255, every ray walks
+    int64_t horizon_rays = 0;        // launched without them
+    cudaEvent_t horizon_done = nullptr;
     std::mutex horizon_mu;
     float* d_xyz = nullptr;          // caller vertices (unscaled) and triangles
     uint32_t* d_idx = nullptr;
@@ -73,6 +75,7 @@ struct sbr_plan {
     sbr::SceneView scene_view{};
     bool multi = false;                      // jobs trace different scenes (JobConst::scene)
     std::vector<sbr::SceneView> scene_views; // multi-scene plans: one per scene
+    std::vector<std::pair<sbr_scene*, int64_t>> scene_rays;  // rays launched on each scene
     sbr::SceneView* d_scenes = nullptr;
 
     std::vector<sbr::Segment> segs;
@@ -164,6 +167,8 @@ sbr_status build_tables(const sbr_scene* const* scenes, const int32_t* job_scene
 
 // Blocks per work item of a segment of a batched sweep, before they are cut down.
 inline int auto_run(int blocks) { return blocks / 1024 < 1 ? 1 : blocks / 1024 > 8 ? 8 : blocks / 1024; }
+// use_horizons for every scene of the plan.
+sbr_status plan_horizons(sbr_plan* pl);
 // Makes the scene's side streams follow the plan's stream, and the plan's follow them.
 sbr_status plan_fork(sbr_plan* pl);
 sbr_status plan_join(sbr_plan* pl);
@@ -178,8 +183,9 @@ sbr_status ensure_fp64(sbr_scene* s);
 // Triangle records, their FP64 twins and boxes (any may be null) from the scene's
 // vertices, on its stream.
 sbr_status write_triangles(sbr_scene* s, GTri* tris, GTri64* tris64, float* box);
-// Computes the scene's horizons unless it holds them, and waits for them.
-sbr_status build_horizons(sbr_scene* s);
+// Tells the scene that `rays` rays are about to be launched on `stream`; computes its
+// horizons there first when they pay by now.
+sbr_status use_horizons(sbr_scene* s, int64_t rays, cudaStream_t stream);
 // Takes them back, in stream order, so that every ray walks (plans that exist see it).
 sbr_status clear_horizons(sbr_scene* s);
 }  // namespace sbr

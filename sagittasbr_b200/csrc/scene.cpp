@@ -71,6 +71,7 @@ void free_scene(sbr_scene* s) {
     for (cudaStream_t q : s->side)
         if (q) cudaStreamDestroy(q);
     if (s->stream) cudaStreamDestroy(s->stream);
+    if (s->horizon_done) cudaEventDestroy(s->horizon_done);
     if (cur >= 0) cudaSetDevice(cur);
     delete s;
 }
@@ -451,9 +452,10 @@ sbr_status sbr_scene_create(const float* xyz, size_t nverts, const uint32_t* tri
             return bail(cuda_fail(e, "8-wide node upload"));
         s->device_bytes += (int64_t)nb8;
     }
-    // (waits for the uploads as well)
-    sbr_status hs = build_horizons(s);
+    sbr_status hs = clear_horizons(s);
     if (hs != SBR_OK) return bail(hs);
+    // plans may launch on the caller's streams: the scene is there when this returns
+    if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) return bail(cuda_fail(e, "scene upload"));
     gpu_tree_free(gt, s->stream);
     if (o.want_fp64 > 0) {
         sbr_status st = ensure_fp64(s);

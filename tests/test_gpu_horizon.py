@@ -1,7 +1,7 @@
 """Horizons only skip walks that return a miss: a scene with horizons traces bit for bit
-like the same scene without them.  A refit to the vertices the scene already has
-recomputes the same boxes and triangles and drops the horizons, and a plan of fewer than
-200 rays per triangle does not bring them back, so that scene walks for every ray."""
+like the same scene without them.  A scene gets them once its sweeps have launched 1,500
+rays per triangle; a refit to the vertices it already has recomputes the same boxes and triangles
+and drops them again.  Plans made before the horizons change read them as well."""
 import numpy as np
 import pytest
 
@@ -48,9 +48,24 @@ def test_horizons_change_nothing(name, prec):
     th, ph = rng.uniform(0.0, 180.0, 7), rng.uniform(0.0, 360.0, 7)
     G = 2.0 * float(np.abs(v).max()) * 1.8
     job = sbr.JobSpec(th, ph, [1e9, 1.7e9, 3e9, 4e9, 6e9, 9e9], 90, 83, G, 6)
-    assert 7 * 90 * 83 < 200 * t.shape[0]
+    # scene b: below 1,500 rays per triangle over all its sweeps (the records do not count)
+    assert 3 * 7 * 90 * 83 < 1500 * t.shape[0]
     with sbr.Scene(v, t, want_fp64=True) as a, sbr.Scene(v, t, want_fp64=True) as b:
-        b.update_vertices(v)
+        n, rays = 1500, 0
+        while rays <= 1500 * t.shape[0]:
+            many = sbr.JobSpec(np.linspace(20.0, 160.0, 5), np.linspace(0.0, 300.0, 5), [1e9], n, n, G, 1)
+            rays += int(sbr.run(a, many).stats[:, 0].sum())
+        if prec == sbr.PREC_FP64:
+            plan = sbr.Plan(a, [job], precision=prec)
+            plan.execute()
+            with_them = plan.results()
+            a.update_vertices(v)
+            plan.execute()  # the same plan, walking
+            np.testing.assert_array_equal(plan.results().field, with_them.field)
+            plan.close()
+            rays = 0
+            while rays <= 1500 * t.shape[0]:
+                rays += int(sbr.run(a, many).stats[:, 0].sum())
         ra, rb = sbr.trace_records(a, job, precision=prec), sbr.trace_records(b, job, precision=prec)
         for key in ("count", "tri", "dist", "normal", "lastdir", "flags"):
             np.testing.assert_array_equal(ra[key], rb[key], err_msg=key)
