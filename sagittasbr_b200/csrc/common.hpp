@@ -103,6 +103,8 @@ struct SceneView {
     const GNode8* __restrict__ nodes8;  // the 8-wide tree of the same leaves, or null
     const int32_t* __restrict__ tie;    // per slot: rank in the reference's walk order, or null
     const unsigned long long* __restrict__ horizon;  // per slot: a byte per octant of directions (horizon.cu)
+    const int32_t* __restrict__ leaf_of;  // with tris64: per slot, 4 * node + child of its leaf
+    float reach;  // at least the largest coordinate of the scene's bounds
 };
 
 // Horizon bytes are multiples of 1 / kHorizonUnit of d.n; 255 is out of any ray's reach.

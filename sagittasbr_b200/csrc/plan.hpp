@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -34,6 +36,7 @@ struct sbr_scene {
     int64_t n_bin_nodes = 0;
     sbr::GTri* d_tris = nullptr;
     sbr::GTri64* d_tris64 = nullptr;
+    int32_t* d_leaf_of = nullptr;    // with d_tris64, in its block: 4 * node + child of each slot's leaf
     int32_t* d_tri_id = nullptr;
     int32_t* d_tie = nullptr;        // exact-tie ranks (coincident faces of opposite winding), or null
     unsigned long long* d_horizon = nullptr;  // per slot: escape elevations by octant (horizon.cu)
@@ -58,7 +61,11 @@ struct sbr_scene {
     float* d_tri_box = nullptr;
     int64_t device_bytes = 0;
 
-    sbr::SceneView view() const { return sbr::SceneView{d_nodes, d_tris, d_tris64, d_tri_id, d_nodes8, d_tie, d_horizon}; }
+    sbr::SceneView view() const {
+        double reach = 0.0;
+        for (int a = 0; a < 3; ++a) reach = std::max(reach, std::max(std::fabs(aabb_lo[a]), std::fabs(aabb_hi[a])));
+        return sbr::SceneView{d_nodes, d_tris, d_tris64, d_tri_id, d_nodes8, d_tie, d_horizon, d_leaf_of, float(1.001 * reach)};
+    }
 };
 
 struct sbr_plan {
@@ -183,6 +190,8 @@ sbr_status ensure_fp64(sbr_scene* s);
 // Triangle records, their FP64 twins and boxes (any may be null) from the scene's
 // vertices, on its stream.
 sbr_status write_triangles(sbr_scene* s, GTri* tris, GTri64* tris64, float* box);
+// 4 * node + child of every slot's leaf, on the scene's stream.
+sbr_status write_leaf_of(sbr_scene* s, int32_t* leaf_of);
 // Tells the scene that `rays` rays are about to be launched on `stream`; computes its
 // horizons there first when they pay by now.
 sbr_status use_horizons(sbr_scene* s, int64_t rays, cudaStream_t stream);

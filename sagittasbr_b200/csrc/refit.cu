@@ -127,7 +127,25 @@ __global__ void k_refit_level(GNode4* nodes, const int32_t* __restrict__ level_n
     }
 }
 
+__global__ void k_leaf_of(const GNode4* __restrict__ nodes, int64_t n, int32_t* __restrict__ leaf_of) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    for (int c = 0; c < 4; ++c) {
+        const int ref = (&nodes[i].child.x)[c];
+        if (ref >= -1) continue;  // inner, or an empty slot
+        const int code = ~ref, first = code >> 4, cnt = code & 15;
+        for (int k = 0; k < cnt; ++k) leaf_of[first + k] = (int32_t)(4 * i + c);
+    }
+}
+
 }  // namespace
+
+sbr_status write_leaf_of(sbr_scene* s, int32_t* leaf_of) {
+    k_leaf_of<<<(unsigned)((s->n_gnodes + kRefitThreads - 1) / kRefitThreads), kRefitThreads, 0, s->stream>>>(
+        s->d_nodes, s->n_gnodes, leaf_of);
+    SBR_CUDA(cudaGetLastError());
+    return SBR_OK;
+}
 
 sbr_status write_triangles(sbr_scene* s, GTri* tris, GTri64* tris64, float* box) {
     const unsigned gt = (unsigned)((s->ntris + kRefitThreads - 1) / kRefitThreads);

@@ -84,20 +84,23 @@ sbr_status ensure_fp64(sbr_scene* s) {
     if (s->d_tris64) return SBR_OK;
     sbr::DeviceGuard device_guard;
     SBR_CUDA(cudaSetDevice(s->device));
-    const size_t bytes = sizeof(GTri64) * (size_t)s->ntris;
-    GTri64* t64 = nullptr;
-    if (pool_alloc(s->device, &t64, bytes) != cudaSuccess)
+    Parts parts;
+    const size_t tri_at = parts.add(sizeof(GTri64) * (size_t)s->ntris), leaf_at = parts.add(sizeof(int32_t) * (size_t)s->ntris);
+    char* t64 = nullptr;
+    if (pool_alloc(s->device, &t64, parts.size()) != cudaSuccess)
         return fail(SBR_ERR_OOM, "allocation of FP64 triangles failed");
     // plans may launch on the caller's streams: the triangles are there when this returns
-    sbr_status st = write_triangles(s, nullptr, t64, nullptr);
+    sbr_status st = write_triangles(s, nullptr, reinterpret_cast<GTri64*>(t64 + tri_at), nullptr);
+    if (st == SBR_OK) st = write_leaf_of(s, reinterpret_cast<int32_t*>(t64 + leaf_at));
     const cudaError_t e = cudaStreamSynchronize(s->stream);
     if (st == SBR_OK && e != cudaSuccess) st = cuda_fail(e, "FP64 triangles");
     if (st != SBR_OK) {
         pool_free(s->device, t64);
         return st;
     }
-    s->d_tris64 = t64;
-    s->device_bytes += (int64_t)bytes;
+    s->d_tris64 = reinterpret_cast<GTri64*>(t64 + tri_at);
+    s->d_leaf_of = reinterpret_cast<int32_t*>(t64 + leaf_at);
+    s->device_bytes += (int64_t)parts.size();
     return SBR_OK;
 }
 
