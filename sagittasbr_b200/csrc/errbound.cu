@@ -63,6 +63,13 @@ constexpr double kPhaseEps = 1.0e-6;
 constexpr double kPhaseExact = 0.05;  // rad: rays with more phase uncertainty are re-traced in FP64
 constexpr double kLambda = 6.0;       // probabilistic bound multiplier (failure below 6e-8)
 
+// A ray bound for the FP64 re-trace, and its mixed term.
+struct Flagged {
+    int32_t seg, i, j;
+    float amp, Lh, Ll;
+};
+constexpr long long kFlaggedMax = 16ll << 20;  // rays of one launch: all of them may be flagged
+
 struct ErrParams {
     SceneView S;
     const Segment* segs;
@@ -70,8 +77,10 @@ struct ErrParams {
     int32_t n_segs;
     const JobConst* jobs;
     const FreqConst* freqs;
-    int64_t n_items;
+    int64_t item_begin, n_items;   // items of this launch: [item_begin, n_items)
     unsigned long long* queue;
+    Flagged* flagged;              // [rays of a launch]
+    unsigned long long* n_flagged;
     double* acc;       // [n_segs][8]: sum amp, sum amp dLs, Q2, Q1, Q0, re-traced rays, rays, -
     double* dfield;    // [n_samples][2]: sum of (FP64 term - mixed term) of the re-traced rays
     float diag;        // scene bounding-box diagonal (m)
@@ -106,13 +115,13 @@ __device__ __forceinline__ bool wt_tri_flag(const GTri& T, F3 o, const WtRay& w,
     }
     const bool inside = !((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f));
     const float det = __fadd_rn(__fadd_rn(U, V), W);
-    // margins: distance (sheared plane) from the ray to each edge line, and t of the plane
-    const float dU = fabsf(U) * rhypotf(cx - bx, cy - by), dV = fabsf(V) * rhypotf(ax - cx, ay - cy),
-                dW = fabsf(W) * rhypotf(bx - ax, by - ay);
     const float T3 = __fmaf_rn(U, az, __fmaf_rn(V, bz, __fmul_rn(W, cz)));
     const float tp = det != 0.0f ? T3 * w.sz / det : 0.0f;
     const bool inRange = tp >= tMin - dt && tp <= tMax + dt;
-    if (inRange) {
+    if (inRange && !amb) {
+        // margins: distance (sheared plane) from the ray to each edge line
+        const float dU = fabsf(U) * rhypotf(cx - bx, cy - by), dV = fabsf(V) * rhypotf(ax - cx, ay - cy),
+                    dW = fabsf(W) * rhypotf(bx - ax, by - ay);
         if (inside) {
             if (fminf(dU, fminf(dV, dW)) < m) amb = true;
         } else {
@@ -175,6 +184,19 @@ __device__ int closest_flag(const SceneView& S, F3 o, F3 d, float tMin, float& t
         hit = tn <= tf * kSlabSlack;
         return tn;
     };
+    auto pop = [&]() {
+        while (sp > 0) {
+            const unsigned long long e = stack[--sp];
+            if (__uint_as_float((unsigned)(e >> 32)) <= tBest + dt) { ref = (int)(unsigned)e; return true; }
+        }
+        return false;
+    };
+    auto push = [&](int r, float t) {
+        if (sp < kStackDepth) stack[sp++] = pack_entry(r, t);
+        else err |= DEV_ERR_STACK;
+    };
+    // nodes until every lane of the warp has a leaf (or is done), then leaves: taking each
+    // lane's leaf as it comes ran the triangle tests on a few lanes at a time (11.6 -> 8.5 ms)
     for (;;) {
         while (ref >= 0) {
             if (++iters > kIterBudget) { err |= DEV_ERR_BUDGET; return -1; }
@@ -186,57 +208,66 @@ __device__ int closest_flag(const SceneView& S, F3 o, F3 d, float tMin, float& t
             float t[4] = {slab(nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, h[0]), slab(nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, h[1]),
                           slab(nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, h[2]), slab(nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, h[3])};
             int c[4] = {ch.x, ch.y, ch.z, ch.w};
-            const float inf = __int_as_float(0x7f800000);
-            for (int k = 0; k < 4; ++k) t[k] = h[k] ? t[k] : inf;
-            sort4(t, c);
-            for (int k = 3; k >= 0; --k)
-                if (t[k] != inf) {
-                    if (sp < kStackDepth) stack[sp++] = pack_entry(c[k], t[k]);
-                    else err |= DEV_ERR_STACK;
+            const int nh = int(h[0]) + int(h[1]) + int(h[2]) + int(h[3]);
+            // the nearest accepted child next, the others pushed, farthest first; where
+            // the nearest lies beyond the closest hit (by the slab's slack) they all do
+            bool enter = false;
+            if (nh == 1) {
+                ref = h[0] ? c[0] : h[1] ? c[1] : h[2] ? c[2] : c[3];
+                enter = (h[0] ? t[0] : h[1] ? t[1] : h[2] ? t[2] : t[3]) <= tBest + dt;
+            } else if (nh > 1) {
+                const float inf = __int_as_float(0x7f800000);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) t[k] = h[k] ? t[k] : inf;
+                sort4(t, c);
+                enter = t[0] <= tBest + dt;
+                if (enter) {
+                    if (nh > 3) push(c[3], t[3]);
+                    if (nh > 2) push(c[2], t[2]);
+                    push(c[1], t[1]);
+                    ref = c[0];
                 }
-            ref = -1;
-            while (sp > 0) {
-                const unsigned long long e = stack[--sp];
-                if (__uint_as_float((unsigned)(e >> 32)) <= tBest + dt) { ref = (int)(unsigned)e; break; }
             }
-            if (ref == -1) return best;
-            while (ref < 0) {
-                if (++iters > kIterBudget) { err |= DEV_ERR_BUDGET; return -1; }
-                const int code = ~ref;
-                const int first = code >> 4, cnt = code & 15;
-                switch (wr.kz) {
-                    case 0: leaf_flag<0>(S.tris, S.tie, first, cnt, o, wr, tMin, m, dt, tBest, best, amb); break;
-                    case 1: leaf_flag<1>(S.tris, S.tie, first, cnt, o, wr, tMin, m, dt, tBest, best, amb); break;
-                    default: leaf_flag<2>(S.tris, S.tie, first, cnt, o, wr, tMin, m, dt, tBest, best, amb); break;
-                }
-                ref = -1;
-                while (sp > 0) {
-                    const unsigned long long e = stack[--sp];
-                    if (__uint_as_float((unsigned)(e >> 32)) <= tBest + dt) { ref = (int)(unsigned)e; break; }
-                }
-                if (ref == -1) return best;
-            }
+            if (!enter && !pop()) return best;
         }
+        do {
+            if (++iters > kIterBudget) { err |= DEV_ERR_BUDGET; return -1; }
+            const int code = ~ref;
+            const int first = code >> 4, cnt = code & 15;
+            switch (wr.kz) {
+                case 0: leaf_flag<0>(S.tris, S.tie, first, cnt, o, wr, tMin, m, dt, tBest, best, amb); break;
+                case 1: leaf_flag<1>(S.tris, S.tie, first, cnt, o, wr, tMin, m, dt, tBest, best, amb); break;
+                default: leaf_flag<2>(S.tris, S.tie, first, cnt, o, wr, tMin, m, dt, tBest, best, amb); break;
+            }
+            if (!pop()) return best;
+        } while (ref < 0);
     }
 }
 
 // One ray: the mixed sweep's path (start_f, then step_f's arithmetic per bounce)
 // with the uncertainty bounds carried along; rays near a decision or with a large
-// phase uncertainty are re-traced with the FP64 sweep's own step and their term
-// differences added to dfield, the others add to the lane's sums of squares.
+// phase uncertainty are listed for the FP64 re-trace, the others add to the lane's sums of
+// squares.
 // Returns the amplitude the sweep adds for the ray (0 when it adds nothing).
-__device__ __forceinline__ float ray_bound(const ErrParams& P, const Segment& G, const JobConst& J, const FreqConst* F,
-                                         int K, double kmax, int i, int j, double& sa, double& s1, double& q1,
+__device__ __forceinline__ float ray_bound(const ErrParams& P, int seg, const Segment& G, const JobConst& J,
+                                         double kmax, int i, int j, bool valid, double& sa, double& s1, double& q1,
                                          double& s0, unsigned& nex, uint32_t& err) {
     RayF r;
-    start_f<SBR_PREC_MIXED>(r, G, J, i, j);
+    r.count = 0;
+    r.o = f3(0, 0, 0);
+    if (valid) start_f<SBR_PREC_MIXED>(r, G, J, i, j);
     float ue = 2.0f * kU * norm1(r.o);  // origin formed in FP64, rounded to FP32
     float ua = 2.0f * kU;                // FP32 direction
     double dL = double(kU * norm1(r.o));
     double dLs = 0.0;  // the part shared by rays seeing the same geometry the same way
     float dnl = 0.0f;
     bool amb = false;
-    for (int b = 0; b < J.max_bounces; ++b) {
+    // one query per step for the whole warp: on their own the lanes drift apart, one in its
+    // first query while another is in its second, and run nearly one at a time (61 looks at
+    // a 200k-triangle ellipsoid, 8.5 -> 3.0 ms)
+    bool walking = valid && J.max_bounces > 0;
+    while (__any_sync(0xffffffffu, walking)) {
+        if (!walking) continue;
         // a ray already bound for the FP64 re-trace needs no more margins: it walks
         // unpadded (its uncertainty can grow to metres after a grazing bounce, and
         // boxes widened that far would open most of the tree)
@@ -245,7 +276,8 @@ __device__ __forceinline__ float ray_bound(const ErrParams& P, const Segment& G,
         const float dt = exact ? 0.0f : 4.0f * m + 4.0f * kU * (norm1(r.o) + P.diag);
         float tB = 1e20f;
         const int slot = closest_flag(P.S, r.o, r.d, 1.0e-3f, tB, m, dt, amb, err);
-        if (slot < 0) break;
+        walking = slot >= 0;
+        if (!walking) continue;
         const GTri T = P.S.tris[slot];
         const F3 n = f3(T.v0.w, T.v1.w, T.v2.w);
         // the step of step_f (ray.cuh), operation for operation
@@ -270,31 +302,15 @@ __device__ __forceinline__ float ray_bound(const ErrParams& P, const Segment& G,
         ue = ue + tB * ua + dtb + 2.0f * kU * norm1(p) + 1.0e-4f * dnrm;
         ua = ua + 2.0f * dnrm + 4.0f * kU;
         dnl = dnrm;
+        walking = r.count < J.max_bounces;
     }
+    if (!valid) return 0.0f;
     const RayOut om = finish_f<SBR_PREC_MIXED>(r, J);
     dLs += ldexp(om.L, -45);  // the FP32 phase pair (ray.cuh, turns_frac)
     dL += ldexp(om.L, -45);
     if (amb || (r.count > 0 && 2.0 * kmax * dL > kPhaseExact)) {
-        // the FP64 sweep's own ray (start_d / step_d) and the exact term differences
-        RayD rd;
-        PolD ed;
-        start_d(rd, G, J, i, j);
-        if (J.max_bounces > 0) {
-            bool done = false;
-            while (!done) done = step_d<false, false>(rd, ed, P.S, J.max_bounces, err, nullptr);
-        }
-        const RayOut od = finish_d(rd, J);
-        for (int k = 0; k < K; ++k) {
-            double re = 0.0, im = 0.0, rm = 0.0, imm = 0.0;
-            if (od.amp != 0.0f) po_term(SBR_PREC_FP64, F[k], od, re, im);
-            if (om.amp != 0.0f) po_term(SBR_PREC_MIXED, F[k], om, rm, imm);
-            re -= rm * F[k].scale;  // mixed terms are summed without k A / (4 pi)
-            im -= imm * F[k].scale;
-            if (re != 0.0 || im != 0.0) {
-                atomicAdd(P.dfield + 2 * (G.sample_base + k), re);
-                atomicAdd(P.dfield + 2 * (G.sample_base + k) + 1, im);
-            }
-        }
+        // left to k_exact: the FP64 walk of a few lanes would hold up the other rays' warps
+        P.flagged[atomicAdd(P.n_flagged, 1ull)] = Flagged{seg, i, j, om.amp, om.Lh, om.Ll};
         ++nex;
     } else if (r.count > 0) {
         sa += double(om.amp);
@@ -306,14 +322,58 @@ __device__ __forceinline__ float ray_bound(const ErrParams& P, const Segment& G,
     return om.amp;
 }
 
-__global__ void __launch_bounds__(kCtaThreads) k_errbound(const ErrParams P) {
+// One flagged ray per lane: the FP64 sweep's own ray (start_d / step_d), a query per step
+// for the whole warp, and per frequency the difference of its term and the mixed one.  As
+// a kernel of its own it runs on full warps: inside k_errbound the flagged rays of a block,
+// a few of its 32, walked while the others waited (61 looks at a 200k-triangle ellipsoid
+// 12.7 -> 11.6 ms; k_exact itself 0.3 ms of the 3.0 of the whole pass).
+__global__ void __launch_bounds__(kCtaThreads, 8) k_exact(const ErrParams P) {
+    constexpr unsigned FULL = 0xffffffffu;
+    uint32_t err = 0;
+    const unsigned long long n = *P.n_flagged;
+    const int lane = threadIdx.x & 31;
+    for (unsigned long long first = blockIdx.x * (unsigned long long)kCtaThreads + (threadIdx.x & ~31); first < n;
+         first += (unsigned long long)gridDim.x * kCtaThreads) {
+        const bool valid = first + lane < n;
+        const Flagged f = P.flagged[valid ? first + lane : first];
+        const Segment& G = P.segs[f.seg];
+        const JobConst J = P.jobs[G.job];
+        const FreqConst* F = P.freqs + J.freq_base;
+        RayD rd;
+        PolD ed;
+        start_d(rd, G, J, f.i, f.j);
+        bool walking = valid && J.max_bounces > 0;
+        while (__any_sync(FULL, walking))
+            if (walking) walking = !step_d<false, false>(rd, ed, P.S, J.max_bounces, err, nullptr);
+        if (!valid) continue;
+        const RayOut od = finish_d(rd, J);
+        RayOut om;
+        om.amp = f.amp;
+        om.Lh = f.Lh;
+        om.Ll = f.Ll;
+        for (int q = 0; q < J.n_freqs; ++q) {
+            double re = 0.0, im = 0.0, rm = 0.0, imm = 0.0;
+            if (od.amp != 0.0f) po_term(SBR_PREC_FP64, F[q], od, re, im);
+            if (om.amp != 0.0f) po_term(SBR_PREC_MIXED, F[q], om, rm, imm);
+            re -= rm * F[q].scale;  // mixed terms are summed without k A / (4 pi)
+            im -= imm * F[q].scale;
+            if (re != 0.0 || im != 0.0) {
+                atomicAdd(P.dfield + 2 * (G.sample_base + q), re);
+                atomicAdd(P.dfield + 2 * (G.sample_base + q) + 1, im);
+            }
+        }
+    }
+    if (err) atomicOr(P.err, err);
+}
+
+__global__ void __launch_bounds__(kCtaThreads, 8) k_errbound(const ErrParams P) {
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     uint32_t err = 0;
     for (;;) {
         long long item = 0;
         if (lane == 0) {
-            item = (long long)atomicAdd(P.queue, 1ull);
+            item = P.item_begin + (long long)atomicAdd(P.queue, 1ull);
             if (item < P.n_items && P.cancel && *P.cancel != 0) {
                 atomicOr(P.err, DEV_ERR_CANCEL);
                 item = P.n_items;
@@ -334,11 +394,9 @@ __global__ void __launch_bounds__(kCtaThreads) k_errbound(const ErrParams P) {
         for (int blk = b0; blk < b1; ++blk) {
             const int i = G.i0 + (blk % G.blocks_x) * kBlockW + (lane % kBlockW);
             const int j = G.j0 + (blk / G.blocks_x) * kBlockH + (lane / kBlockW);
-            float am = 0.0f;
-            if (i < G.i0 + G.ni && j < G.j0 + G.nj) {
-                am = ray_bound(P, G, J, F, J.n_freqs, kmax, i, j, sa, s1, q1, s0, nex, err);
-                ++nray;
-            }
+            const bool valid = i < G.i0 + G.ni && j < G.j0 + G.nj;
+            const float am = ray_bound(P, seg, G, J, kmax, i, j, valid, sa, s1, q1, s0, nex, err);
+            nray += valid;
             // the block's FP32 partial sums: n_b terms, every partial within A_b
             double ab = double(fabsf(am));
 #pragma unroll
@@ -395,11 +453,17 @@ extern "C" sbr_status sbr_error_bound(sbr_scene* s, const sbr_job* jobs, size_t 
     double* d_acc = nullptr;
     double* d_dfield = nullptr;
     unsigned long long* d_queue = nullptr;
+    std::vector<int32_t> run_blocks;  // the most blocks an item of each segment has
+    for (const Segment& g : p->segs) run_blocks.push_back(g.parts > 1 ? g.part_blocks : g.blocks_per_item);
     std::vector<double> acc(8 * (size_t)std::max<int64_t>(p->n_segs, 1), 0.0);
     std::vector<double> dfield(2 * (size_t)std::max<int64_t>(p->n_samples, 1), 0.0);
     Parts parts;
     const size_t acc_at = parts.add(acc.size() * sizeof(double)), df_at = parts.add(dfield.size() * sizeof(double)),
-                 queue_at = parts.add(sizeof(unsigned long long));
+                 queue_at = parts.add(2 * sizeof(unsigned long long)), zero_b = parts.add(0);
+    // a launch takes as many items as the list of flagged rays has room for
+    const long long run = std::max<int64_t>(1, p->n_items > 0 ? *std::max_element(run_blocks.begin(), run_blocks.end()) : 1);
+    const long long per_launch = std::max<long long>(1, std::min<long long>(p->n_items, kFlaggedMax / (32 * run)));
+    const size_t flag_at = parts.add((size_t)(per_launch * run * 32) * sizeof(Flagged));
     char* block = nullptr;
     cudaError_t e = pool_alloc(p->device, &block, parts.size());
     if (e != cudaSuccess) st = fail(SBR_ERR_OOM, "error-bound accumulators");
@@ -407,7 +471,7 @@ extern "C" sbr_status sbr_error_bound(sbr_scene* s, const sbr_job* jobs, size_t 
         d_acc = reinterpret_cast<double*>(block + acc_at);
         d_dfield = reinterpret_cast<double*>(block + df_at);
         d_queue = reinterpret_cast<unsigned long long*>(block + queue_at);
-        e = cudaMemsetAsync(block, 0, parts.size(), p->stream);
+        e = cudaMemsetAsync(block, 0, zero_b, p->stream);
         if (e != cudaSuccess) st = cuda_fail(e, "error-bound clear");
     }
     if (st == SBR_OK && p->n_items > 0) {
@@ -419,8 +483,9 @@ extern "C" sbr_status sbr_error_bound(sbr_scene* s, const sbr_job* jobs, size_t 
         P.seg_item_base = p->d_seg_base;
         P.n_segs = (int32_t)p->n_segs;
         P.jobs = p->d_jobs;
-        P.n_items = p->n_items;
         P.queue = d_queue;
+        P.n_flagged = d_queue + 1;
+        P.flagged = reinterpret_cast<Flagged*>(block + flag_at);
         P.acc = d_acc;
         const double dx = s->aabb_hi[0] - s->aabb_lo[0], dy = s->aabb_hi[1] - s->aabb_lo[1],
                      dz = s->aabb_hi[2] - s->aabb_lo[2];
@@ -431,9 +496,17 @@ extern "C" sbr_status sbr_error_bound(sbr_scene* s, const sbr_job* jobs, size_t 
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_errbound, kCtaThreads, 0);
         if (e != cudaSuccess) st = cuda_fail(e, "occupancy");
         if (st == SBR_OK) {
-            const long long grid = std::min<long long>((long long)std::max(occ, 1) * p->num_sms, (p->n_items + 3) / 4);
-            k_errbound<<<(unsigned)std::max(grid, 1LL), kCtaThreads, 0, p->stream>>>(P);
-            e = cudaGetLastError();
+            for (long long at = 0; at < p->n_items && e == cudaSuccess; at += per_launch) {
+                P.item_begin = at;
+                P.n_items = std::min<long long>(p->n_items, at + per_launch);
+                if (at > 0) e = cudaMemsetAsync(d_queue, 0, 2 * sizeof(unsigned long long), p->stream);
+                if (e != cudaSuccess) break;
+                const long long grid = std::min<long long>((long long)std::max(occ, 1) * p->num_sms, (P.n_items - at + 3) / 4);
+                k_errbound<<<(unsigned)std::max(grid, 1LL), kCtaThreads, 0, p->stream>>>(P);
+                const long long most = (per_launch * run * 32 + kCtaThreads - 1) / kCtaThreads;
+                k_exact<<<(unsigned)std::min<long long>(most, 8ll * p->num_sms), kCtaThreads, 0, p->stream>>>(P);
+                e = cudaGetLastError();
+            }
             if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
             if (e != cudaSuccess) st = cuda_fail(e, "error-bound pass");
         }
