@@ -33,6 +33,7 @@ struct TraceParams {
     int32_t k_begin, k_count;      // frequency sub-range of every job (k_count 0 -> all)
     int32_t count_stats;
     int32_t n_rep;                 // accumulator replicas per sample
+    int32_t lanes_log2;            // rays a warp takes at a time: 32, or fewer in small launches
     const JobConst* jobs;
     const FreqConst* freqs;
     int64_t item_begin, item_end;  // items handled by this launch
@@ -197,6 +198,11 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
         item = __shfl_sync(FULL, item, 0);
         if (item >= P.item_end) break;
         ++iter;
+        // small launches: 2^sub items of one block share it, a warp taking the block's next
+        // 32 >> sub rays on as many lanes
+        const int sub = 5 - P.lanes_log2;
+        const int part = int(item & ((1 << sub) - 1));
+        item >>= sub;
 
         const int seg = find_segment(P.seg_item_base, P.n_segs, item);
         const Segment& G = P.segs[seg];
@@ -207,7 +213,8 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
         const FreqConst* F = P.freqs + J.freq_base + kb;
         const Run run = item_run(G, item, PART);
         const int b0 = run.first;
-        const int nslots = run.count * 32;
+        const int nslots = min(run.count * 32, sub == 0 ? INT_MAX : (part + 1) << P.lanes_log2);
+        const bool usable = (lane >> P.lanes_log2) == 0;
         const int i_end = G.i0 + G.ni, j_end = G.j0 + G.nj;
         const int KC = K * NPOL;  // channels of this item
 
@@ -229,11 +236,12 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
         bool active = false;
         int queries = 0;
         sbr_ray_record* rec = nullptr;
-        int next = 0;  // next slot of the item to hand out (same value in every lane)
+        // next slot of the item to hand out (same value in every lane)
+        int next = part << P.lanes_log2;
 
         auto refill = [&]() {
             for (;;) {
-                const unsigned need = __ballot_sync(FULL, !active);
+                const unsigned need = __ballot_sync(FULL, usable && !active);
                 if (need == 0 || next >= nslots) break;
                 if (!REC && P.tile_cnt != nullptr && need == FULL) {
                     // full blocks whose tile no triangle reaches: all 32 rays miss their
@@ -253,7 +261,7 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
                     if (next >= nslots) break;
                 }
                 const int s = next + __popc(need & ((1u << lane) - 1u));
-                if (!active && s < nslots) {
+                if (usable && !active && s < nslots) {
                     const int blk = b0 + (s >> 5), l = s & 31;
                     const int i = G.i0 + (blk % G.blocks_x) * kBlockW + (l % kBlockW);
                     const int j = G.j0 + (blk / G.blocks_x) * kBlockH + (l / kBlockW);
@@ -975,11 +983,30 @@ sbr_status tile_raster(sbr_plan* pl, const sbr_plan::Chunk& ch, cudaStream_t st,
 
 }  // namespace
 
+// Rays a warp takes at a time in a launch of `items`, as a power of two.  A launch that
+// leaves most warps without a block lasts as long as one warp needs for a block, and that
+// is as long as its lanes' walks take together where they part: such a launch shares a
+// block between up to 8 warps of 4 rays, while all of them fit on the chip at once.
+// Measured on B200 with 32 rays / at most 16 / 32 / 64 warps an SM, us: one look at a
+// 20k-triangle sphere (145 blocks) 54 / 38 / 38 / 37, four 59 / 52 / 52 / 49, thirty (4,350)
+// 92 / 92 / 93 / 107, one at a 200k-triangle ellipsoid (555) 210 / 149 / 121 / 124, FP64
+// sphere 69 / 46 / 47 / 46, plates with six bounces 285 / 285 / 234 / 196.
+// Blocks whose terms are added in FP32 first (more than kRegK mixed channels) stay whole.
+static int lanes_log2(const sbr_plan* pl, int channels, long long items) {
+    if (pl->prec == SBR_PREC_MIXED && channels > kRegK) return 5;
+    for (const Segment& g : pl->segs)
+        if (g.blocks_per_item != 1) return 5;
+    int lg = 5;
+    while (lg > 2 && (items << (6 - lg)) <= 32ll * pl->num_sms) --lg;
+    return lg;
+}
+
 sbr_status plan_launch(sbr_plan* pl, bool records, sbr_ray_record* d_records) {
     const bool pol = pl->pol == SBR_POL_HHVV && !records;
     const int npol = pol ? 2 : 1;
     const bool batched = pl->mode == SBR_MODE_BATCHED || records;
-    const void* fn = pick_kernel(pl->prec, (batched ? pl->k_max : 1) * npol, records, pol, pl->multi,
+    const int channels = (batched ? pl->k_max : 1) * npol;
+    const void* fn = pick_kernel(pl->prec, channels, records, pol, pl->multi,
                                  pl->scene_view.nodes8 != nullptr);
     TraceParams p{};
     p.segpol = pl->d_segpol;
@@ -989,6 +1016,7 @@ sbr_status plan_launch(sbr_plan* pl, bool records, sbr_ray_record* d_records) {
     p.seg_item_base = pl->d_seg_base;
     p.n_segs = (int32_t)pl->n_segs;
     p.n_rep = kAccReplicas;
+    p.lanes_log2 = 5;
     p.jobs = pl->d_jobs;
     p.freqs = pl->d_freqs;
     p.acc = pl->d_acc;
@@ -1010,6 +1038,7 @@ sbr_status plan_launch(sbr_plan* pl, bool records, sbr_ray_record* d_records) {
             p.count_stats = 1;
             p.zbuf = pl->d_zbuf;
             p.tile_cnt = pl->d_tile_cnt;
+            p.lanes_log2 = lanes_log2(pl, channels, pl->n_items);
             for (size_t c = 0; c < pl->chunks.size(); ++c) {
                 const sbr_plan::Chunk& ch = pl->chunks[c];
                 if (ch.tiles > 0) {
@@ -1017,10 +1046,10 @@ sbr_status plan_launch(sbr_plan* pl, bool records, sbr_ray_record* d_records) {
                     if (s != SBR_OK) return s;
                 }
                 if (ch.item_end > ch.item_begin) {
-                    p.item_begin = ch.item_begin;
-                    p.item_end = ch.item_end;
+                    p.item_begin = ch.item_begin << (5 - p.lanes_log2);
+                    p.item_end = ch.item_end << (5 - p.lanes_log2);
                     p.queue = pl->d_queue + 1 + pl->n_samples + c;
-                    const int grid = (int)std::min<long long>(pl->persistent_grid, (ch.item_end - ch.item_begin + 3) / 4);
+                    const int grid = (int)std::min<long long>(pl->persistent_grid, (p.item_end - p.item_begin + 3) / 4);
                     sbr_status s = launch_trace(fn, grid, st, p);
                     if (s != SBR_OK) return s;
                     ++launches;
@@ -1030,10 +1059,11 @@ sbr_status plan_launch(sbr_plan* pl, bool records, sbr_ray_record* d_records) {
             p.k_begin = 0;
             p.k_count = 0;
             p.count_stats = 1;
+            p.lanes_log2 = lanes_log2(pl, channels, pl->n_items);
             p.item_begin = 0;
-            p.item_end = pl->n_items;
+            p.item_end = pl->n_items << (5 - p.lanes_log2);
             p.queue = pl->d_queue;
-            const long long warps_needed = pl->n_items;
+            const long long warps_needed = p.item_end;
             const int grid = (int)std::min<long long>(pl->persistent_grid, (warps_needed + 3) / 4);
             sbr_status s = launch_trace(fn, grid, st, p);
             if (s != SBR_OK) return s;
@@ -1253,6 +1283,7 @@ extern "C" sbr_status sbr_run_noalloc(sbr_scene* s, const sbr_job* job, double* 
         p.k_count = 0;
         p.count_stats = 1;
         p.n_rep = 1;
+        p.lanes_log2 = 5;
         p.jobs = &D->tables.job;
         p.freqs = D->tables.freqs;
         p.item_begin = 0;

@@ -32,3 +32,21 @@ def test_automatic_items_equal_whole_runs(nx, ny, run, prec, nf):
     np.testing.assert_array_equal(a.stats, b.stats)
     # FP64 sums of the same terms: a few roundings of each partial sum
     assert np.abs(a.field - b.field).max() <= 1e-12 * np.abs(b.field).max()
+
+
+@pytest.mark.parametrize("nf", [1, 3, 4, 5, 40])
+@pytest.mark.parametrize("prec", [sbr.PREC_MIXED, sbr.PREC_FP32, sbr.PREC_FP64])
+@pytest.mark.parametrize("nx, ny", [(9, 5), (33, 31), (64, 64), (130, 127), (200, 190)])
+def test_small_launch_equals_its_part_of_a_large_one(nx, ny, prec, nf):
+    """One angle alone (its blocks shared by several warps) and among 80 (whole blocks)."""
+    v, t = M.plate_cluster(12, 5, seed=4)
+    fr = np.linspace(1e9, 3e9, nf)
+    ph = np.linspace(0.0, 350.0, 80)
+    with sbr.Scene(v, t, want_fp64=True) as s:
+        many = sbr.run(s, sbr.JobSpec(np.full(80, 65.0), ph, fr, nx, ny, 2.2, 4), precision=prec)
+        for k in (0, 37, 79):
+            one = sbr.run(s, sbr.JobSpec([65.0], ph[k:k + 1], fr, nx, ny, 2.2, 4), precision=prec)
+            np.testing.assert_array_equal(one.stats[0], many.stats[k])
+            m = many.field[k * nf:(k + 1) * nf]
+            # FP64 sums of the same terms, and roundings to units of 2^-60 of the field's bound
+            assert np.abs(one.field - m).max() <= 1e-12 * np.abs(many.field).max()
