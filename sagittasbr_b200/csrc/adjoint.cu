@@ -87,7 +87,7 @@ __device__ __forceinline__ void adjoint_ray(const AdjointParams& P, const Segmen
         r.count = 0;
         if (valid) start_f<PREC>(r, G, J, i, j);
         while (__any_sync(FULL, walking))
-            if (walking) walking = !step_f<PREC, true, false>(r, e, P.S, J.max_bounces, err, &rec, nullptr, nullptr);
+            if (walking) walking = !step_f<PREC, true, false, false, false, true>(r, e, P.S, J.max_bounces, err, &rec, nullptr, nullptr);
         n = valid ? r.count : 0;
     }
     if (n == 0) return;
@@ -188,10 +188,12 @@ __device__ __forceinline__ void adjoint_ray(const AdjointParams& P, const Segmen
     }
 }
 
-// 6 resident CTAs per SM (80 registers): measured 8 % faster on B200 than the
-// unconstrained 128-register build despite the spills.
+// 9 resident CTAs per SM (56 registers): the walk waits on node loads, and resident warps
+// count for more than the spills.  Measured on B200 at 6 / 8 / 9 / 10 / 12, ms a gradient of
+// 121 looks at 200k triangles: jittered ellipsoid 4.98 / 4.64 / 4.42 / 4.61 / 6.35, smooth
+// 3.58 / 3.23 / 3.14 / 3.30 / 4.33 (6 with the scalar slab planes; at 8 those gave 4.61 / 3.31).
 template <int PREC>
-__global__ void __launch_bounds__(kCtaThreads, 6) k_adjoint(const AdjointParams P) {
+__global__ void __launch_bounds__(kCtaThreads, 9) k_adjoint(const AdjointParams P) {
     constexpr unsigned FULL = 0xffffffffu;
     double gk[kAdjMaxK];  // this lane's dLoss/dk of the current item (local memory)
     const int lane = threadIdx.x & 31;

@@ -134,7 +134,8 @@ constexpr unsigned long long kZWalk = 0xfffffffe00000000ull;
 // The first query is read from the first-hit buffer when there is one (a tile no
 // triangle reaches has no entries there).
 // SPEC: the speculative closest-hit walk, entered by all lanes of `mask` together.
-template <int PREC, bool REC, bool POL, bool W8 = false, bool SPEC = false>
+// F2: slab planes two-wide (the sweep's record and polarised kernels have no registers for it).
+template <int PREC, bool REC, bool POL, bool W8 = false, bool SPEC = false, bool F2 = !REC && !POL>
 __device__ __forceinline__ bool step_f(RayF& r, PolF& e, const SceneView& S, int maxB, uint32_t& err,
                                        sbr_ray_record* rec, const unsigned long long* zbuf, const uint32_t* tile_cnt,
                                        unsigned mask = 0u) {
@@ -154,7 +155,7 @@ __device__ __forceinline__ bool step_f(RayF& r, PolF& e, const SceneView& S, int
         static_assert(PREC == SBR_PREC_MIXED && !REC && !POL, "the 8-wide walk is the mixed scalar sweep's");
         slot = Walker8::closest(S, r.o, r.d, 1.0e-3f, tB, err);
     } else {
-        slot = Walker<false>::closest<PREC == SBR_PREC_MIXED, !REC && !POL>(S, r.o, r.d, 1.0e-3f, tB, err);
+        slot = Walker<false>::closest<PREC == SBR_PREC_MIXED, F2>(S, r.o, r.d, 1.0e-3f, tB, err);
     }
     if (slot < 0) return true;
     const GTri* T = S.tris + slot;
