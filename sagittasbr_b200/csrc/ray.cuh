@@ -134,8 +134,8 @@ constexpr unsigned long long kZWalk = 0xfffffffe00000000ull;
 // The first query is read from the first-hit buffer when there is one (a tile no
 // triangle reaches has no entries there).
 // SPEC: the speculative closest-hit walk, entered by all lanes of `mask` together.
-// F2: slab planes two-wide (the sweep's record and polarised kernels have no registers for it).
-template <int PREC, bool REC, bool POL, bool W8 = false, bool SPEC = false, bool F2 = !REC && !POL>
+// F2: slab planes two-wide (see Walker<false>).
+template <int PREC, bool REC, bool POL, bool W8 = false, bool SPEC = false, bool F2 = !REC>
 __device__ __forceinline__ bool step_f(RayF& r, PolF& e, const SceneView& S, int maxB, uint32_t& err,
                                        sbr_ray_record* rec, const unsigned long long* zbuf, const uint32_t* tile_cnt,
                                        unsigned mask = 0u) {
