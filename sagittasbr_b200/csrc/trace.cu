@@ -56,24 +56,32 @@ constexpr int kRegK = 4;     // per-lane accumulation up to this many channels
 // (scalar plans) or its (frequency, polarisation) pairs, channel 2k + p (HHVV plans).
 //   EPI_LANE1, EPI_LANE4: every lane sums the terms of its own rays for up to 1 / 4
 //                         channels (registers sized to the plan's channel count)
-//   EPI_T64, EPI_T128:    lanes own channels lane, lane + 32, ...; each finished ray
-//                         is broadcast to the warp (up to 64 / 128 channels)
-enum : int { EPI_LANE1 = 0, EPI_LANE4 = 1, EPI_T64 = 2, EPI_T128 = 3 };
+//   EPI_T32 / T64 / T128: lanes own channels lane, lane + 32, ...; each finished ray
+//                         is broadcast to the warp (up to 32 / 64 / 128 channels)
+// A channel's terms are added in the same order in all three, so the layout changes no
+// field; it sets the registers and the columns a broadcast ray is offered to.  Up to 32
+// channels EPI_T32 against EPI_T64, ms on B200: 8 scalar frequencies, aircraft of 537k
+// triangles 12.99 -> 12.15, trihedral 25.49 -> 23.76, ellipsoid 3.23 -> 3.08, sphere
+// 0.545 -> 0.513; 16 frequencies HHVV 13.81 -> 12.87, 27.59 -> 25.90, 3.34 -> 3.18,
+// 0.572 -> 0.535.
+enum : int { EPI_LANE1 = 0, EPI_LANE4 = 1, EPI_T32 = 2, EPI_T64 = 3, EPI_T128 = 4 };
 template <int EPI>
 struct Epi {
-    static constexpr bool kTransposed = EPI >= EPI_T64;
-    static constexpr int kAcc = EPI == EPI_LANE1 ? 1 : EPI == EPI_LANE4 ? 4 : EPI == EPI_T64 ? 2 : 4;
+    static constexpr bool kTransposed = EPI >= EPI_T32;
+    static constexpr int kAcc = EPI == EPI_LANE1 || EPI == EPI_T32 ? 1 : EPI == EPI_T64 ? 2 : 4;
     static constexpr int kChannels = kTransposed ? 32 * kAcc : kAcc;
 };
 inline int pick_epi(int channels) {
-    return channels <= 1 ? EPI_LANE1 : channels <= kRegK ? EPI_LANE4 : channels <= 64 ? EPI_T64 : EPI_T128;
+    return channels <= 1 ? EPI_LANE1 : channels <= kRegK ? EPI_LANE4 : channels <= 32 ? EPI_T32
+           : channels <= 64 ? EPI_T64 : EPI_T128;
 }
 // Resident CTAs (of 4 warps) per SM the kernels are register-budgeted for, by
 // epilogue layout: the walk is latency-bound (node loads from L1/L2), so resident
 // warps matter, but the wide layouts hold more state.  Measured on B200: per-lane
 // layouts, trihedral (1 channel) 50,993 / 49,455 / 47,565 samples/s at 8 / 7 / 6
 // CTAs (64 / 72 / 80 registers); lane-owned layouts, aircraft (64 channels)
-// 13,180 / 13,499 / 12,948.  SBR_TRACE_CTAS_PER_SM (build flag) overrides both.
+// 13,180 / 13,499 / 12,948; one column of them (EPI_T32), aircraft of 537k triangles at
+// 8 frequencies 12.15 / 12.36 ms at 8 / 7.  SBR_TRACE_CTAS_PER_SM (build flag) overrides both.
 // SBR_TRACE_SPECULATIVE=1 (build flag): the mixed scalar sweep walks with the
 // speculative closest-hit walk (trace.cuh) instead of the per-lane while-while one.
 #ifndef SBR_TRACE_SPECULATIVE
@@ -885,6 +893,7 @@ const void* pick_epi_kernel(int epi) {
     switch (epi) {
         case EPI_LANE1: return kernel_ptr<PREC, EPI_LANE1, REC, POL, MULTI>();
         case EPI_LANE4: return kernel_ptr<PREC, EPI_LANE4, REC, POL, MULTI>();
+        case EPI_T32: return kernel_ptr<PREC, EPI_T32, REC, POL, MULTI>();
         case EPI_T64: return kernel_ptr<PREC, EPI_T64, REC, POL, MULTI>();
         default: return kernel_ptr<PREC, EPI_T128, REC, POL, MULTI>();
     }
@@ -901,6 +910,7 @@ const void* pick_kernel(int prec, int channels, bool rec, bool pol, bool multi =
         switch (epi) {
             case EPI_LANE1: return kernel_ptr<SBR_PREC_MIXED, EPI_LANE1, false, false, false, true>();
             case EPI_LANE4: return kernel_ptr<SBR_PREC_MIXED, EPI_LANE4, false, false, false, true>();
+            case EPI_T32: return kernel_ptr<SBR_PREC_MIXED, EPI_T32, false, false, false, true>();
             case EPI_T64: return kernel_ptr<SBR_PREC_MIXED, EPI_T64, false, false, false, true>();
             default: return kernel_ptr<SBR_PREC_MIXED, EPI_T128, false, false, false, true>();
         }
