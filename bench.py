@@ -283,10 +283,17 @@ class CpuReference:
     its release flags) on all host cores, timed on uniform samples of the sweep's ray
     rows; the reference tree is built once and not timed."""
 
+    MISSING = "oracle/_ref/libsbrref32_fast.so not built (make -C oracle with the reference)"
+
+    @staticmethod
+    def available() -> bool:
+        from oracle import oracle as O
+        return O.ref_available("32fast")
+
     def __init__(self, w, threads: int = 0):
         from oracle import oracle as O
-        if not O.ref_available("32fast"):
-            raise RuntimeError("oracle/_ref/libsbrref32_fast.so is not built (make -C oracle with the reference)")
+        if not self.available():
+            raise RuntimeError(self.MISSING)
         self.w, self.threads = w, threads or (os.cpu_count() or 1)
         self.scene = O.RefScene(w["verts"], w["tris"], kind="32fast")
         self.rng = np.random.default_rng(7)
@@ -365,6 +372,9 @@ def run_reference_arm(args):
     ray rows; rank 0 alone runs under torchrun."""
     ws, rank, _ = dist_env()
     if rank != 0:
+        return 0
+    if not CpuReference.available():
+        print(json.dumps({"impl": "reference", "unavailable": CpuReference.MISSING}))
         return 0
     w = workload(args.workload)
     ref = CpuReference(w)
@@ -793,7 +803,9 @@ def main():
     peak = fp32_peak_tflops(torch)
     if not args.no_ref_gpu and ws == 1 and args.angles == 0 and args.workload in REF_GPU_SAMPLES:
         refg = ref_gpu_leg(w, sbr, scene, value)
-    if not args.no_cpu and ws == 1:
+    if not args.no_cpu and ws == 1 and not CpuReference.available():
+        cpu = {"unavailable": CpuReference.MISSING}
+    elif not args.no_cpu and ws == 1:
         c = CpuReference(w).sample(10.0)
         cpu = {"value": c["value"], "unit": "samples/s", "cores": os.cpu_count(), "kind": "reference",
                "sample": c["sample"], "mray_bounces_per_s": c["mray_bounces_per_s"], "rays_per_s": c["rays_per_s"]}
