@@ -136,6 +136,7 @@ struct __align__(16) Segment {
     // t = pt[0..2].P + pt[3] (pixel (i, j) is centred at s = i, t = j)
     double ps[4], pt[4];
     float margin;         // pixels by which the first-hit raster widens projected triangles
+    float finer;          // the angle's accumulator units per unit of its job (a power of two)
     int64_t zbase;        // first first-hit buffer entry of this segment within its chunk (32 tbase;
                           // entries are tile-major: tile, then lane of the 4 x 8 block)
 };
@@ -169,7 +170,7 @@ struct JobConst {
 struct FreqConst {
     double k;
     double scale;         // k * rayArea / (4 pi)
-    double quantum;       // field value of one accumulator unit
+    double quantum;       // field value of one accumulator unit of the job (an angle's: / finer)
     double inv_quantum;
     double turns;         // k / pi
     float kf;

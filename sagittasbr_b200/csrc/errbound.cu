@@ -544,7 +544,7 @@ extern "C" sbr_status sbr_error_bound(sbr_scene* s, const sbr_job* jobs, size_t 
                 const double shared = a * ((A[0] > 0.0 ? 2.0 * F.k * A[1] / A[0] : 0.0) + kPhaseEps);
                 const double E = std::hypot(dfield[2 * smp], dfield[2 * smp + 1]) + shared +
                                  kLambda * F.scale * (2.0 * F.k * std::sqrt(A[3]) + std::sqrt(A[4])) +
-                                 double(items + 1) * F.quantum + kLambda * F.scale * double(kU) * std::sqrt(A[2]);
+                                 4.0 * double(items + 1) * F.quantum + kLambda * F.scale * double(kU) * std::sqrt(A[2]);
                 if (err_field) err_field[smp] = E;
                 if (err_db) {
                     const double db = 10.0 * std::log10(std::max(4.0 * M_PI * a * a, 1e-10));

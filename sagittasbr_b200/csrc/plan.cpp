@@ -208,9 +208,11 @@ sbr_status build_tables(const sbr_scene* const* scenes, const int32_t* job_scene
             float lambdaf = 299792458.0f / float(J.freq_hz[f]);
             fc.kf = 2.0f * float(M_PI) / lambdaf;
             fc.scalef = fc.kf * areaf / (4.0f * float(M_PI));
-            // |field| <= rays * k A/(4 pi) * 2 * max(1,R)^maxB; 2^60 units cover it with margin
+            // |field| <= rays * k A/(4 pi) * 2 * max(1,R)^maxB, in 2^62 units; every term is
+            // rounded to a unit, and the int64 sums (below 2^63) have a factor of two over
+            // for the terms' own roundings
             double bound = double(int64_t(J.nx) * int64_t(J.ny)) * std::max(fc.scale, double(fc.scalef)) * 2.0 * rmax;
-            double q = bound / 1152921504606846976.0;  // 2^60
+            double q = bound / 4611686018427387904.0;  // 2^62
             if (!std::isfinite(q) || !(q > 0))
                 return fail(SBR_ERR_TOO_LARGE, "field bound overflows (reflection_const^max_bounces too large)");
             fc.quantum = q;
@@ -302,7 +304,13 @@ sbr_status build_tables(const sbr_scene* const* scenes, const int32_t* job_scene
             sample += J.n_freqs;
             tot.n_rays_clipped += (int64_t)g.ni * g.nj;
             tot.n_rays_grid += (int64_t)J.nx * J.ny;
-            if (!sink.segment(g, item, quantum, (int)J.n_freqs))
+            // only the clipped rectangle's rays add to the field: units as much finer
+            g.finer = 1.0f;
+            const int64_t rays = std::max<int64_t>(1, (int64_t)g.ni * g.nj);
+            while (double(2.0f * g.finer) * double(rays) <= double(int64_t(J.nx) * int64_t(J.ny))) g.finer *= 2.0f;
+            double units[128];
+            for (int64_t f = 0; f < J.n_freqs; ++f) units[f] = quantum[f] / double(g.finer);
+            if (!sink.segment(g, item, units, (int)J.n_freqs))
                 return fail(SBR_ERR_TOO_LARGE, "table capacity exceeded (angles or samples)");
             tot.n_segs += 1;
         }

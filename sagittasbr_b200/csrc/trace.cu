@@ -2,13 +2,13 @@
 //
 // One work item = a run of 4x8-ray blocks of one (job, angle) segment, owned by
 // one warp.  Warps take items from a device queue (persistent grid), trace one
-// 4x8 block of parallel rays at a time through every bounce (trace.cuh), and fold
-// the PO exit-ray term of every frequency of the job into per-lane FP64 sums.  At
-// the end of an item the warp reduces them in a fixed order and adds the total, quantised to a per-frequency fixed-point unit,
-// to int64 accumulators with atomicAdd.  Integer addition is associative, so the
-// field is bitwise reproducible whatever order the items finish in (the reference
-// adds FP32 block sums with float atomics, src/cuda/poKernels.cu:118-120, whose
-// order changes run to run).
+// 4x8 block of parallel rays at a time through every bounce (trace.cuh), and round
+// the PO exit-ray term of every frequency of the job to a fixed-point unit of the
+// sample, which each lane sums in int64.  At the end of an item the warp adds its sums
+// to the sample's int64 accumulators with atomicAdd.  Integer addition is associative,
+// so the field is bitwise reproducible whatever order the items finish in and however a
+// sweep is cut into items, launches and plans (the reference adds FP32 block sums with
+// float atomics, src/cuda/poKernels.cu:118-120, whose order changes run to run).
 //
 // Replaces launchRaysMultiBounce + integratePoMultiBounce (src/cuda/rtKernels.cu:105-158,
 // src/cuda/poKernels.cu:66-121) and the per-angle loop of runSweep
@@ -151,25 +151,26 @@ __device__ __forceinline__ void po_term_pol(int prec, const FreqConst& F, double
     }
 }
 
-// Accumulator units per unit of a lane sum: MIXED sums leave out k A / (4 pi).
+// Accumulator units per unit of a term: MIXED terms leave out k A / (4 pi).
 template <int PREC>
-__device__ __forceinline__ double fold_factor(const FreqConst& F) {
-    return PREC == SBR_PREC_MIXED ? F.scale * F.inv_quantum : F.inv_quantum;
+__device__ __forceinline__ double units_per(const FreqConst& F, const Segment& G) {
+    return double(G.finer) * (PREC == SBR_PREC_MIXED ? F.scale * F.inv_quantum : F.inv_quantum);
 }
 
-__device__ __forceinline__ void add_fixed(unsigned long long* acc, double v, double invQ) {
-    const long long q = __double2ll_rn(v * invQ);
+__device__ __forceinline__ void add_fixed(unsigned long long* acc, long long q) {
     if (q != 0) atomicAdd(acc, (unsigned long long)q);
 }
 
 // Warp-persistent sweep kernel.  Every warp independently takes a work item (a
 // run of 4x8-ray blocks of one (job, angle) segment) and traces it one block at a
 // time, all lanes at the same bounce (no CTA-wide barrier anywhere).  Each lane
-// folds the PO terms of its finished rays into FP64 sums (MIXED lane-owned
-// layouts: through FP32 partial sums of one 4x8 block); at the end of the item
-// the warp reduces them in a fixed order and adds the total, as int64 fixed
-// point, to one of the segment's accumulator replicas.  Which lane takes which
-// ray depends only on the item, so every sum is reproducible bit for bit.
+// rounds the PO term of a finished ray (MIXED lane-owned layouts: the FP32 sum of one
+// group of 32 rays) to the sample's fixed-point unit and adds it to an int64 sum; at the
+// end of the item the warp adds its sums to one of the segment's accumulator replicas.
+// No floating-point sum outlives a ray or a group, and groups form within runs of blocks
+// that the angle alone defines (item_run), so neither the cut into items nor the warps
+// that share a block change a field: an angle alone, in a shard and in any plan of the
+// same options has the same bits.
 template <int PREC, int EPI, bool REC, bool POL, bool MULTI, bool W8 = false>
 __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(const TraceParams P) {
     constexpr unsigned FULL = 0xffffffffu;
@@ -180,17 +181,16 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
     const int lane = threadIdx.x & 31;
     const int warp_global = (int)((blockIdx.x * (unsigned)kCtaThreads + threadIdx.x) >> 5);
     // MIXED lane-owned epilogues sum each block's terms (at most 32 per channel) in
-    // FP32 and add the block partials to the FP64 sums: the FP32 pair phase, one
-    // sine / cosine and two FMAs per (ray, channel), no conversions.  Their FP64
-    // sums stay in registers (measured on B200 against shared memory: aircraft
-    // 14,198 vs 14,035 samples/s, HH + VV aircraft 11,689 vs 11,268).  The FP32 /
-    // FP64 polarised lane-owned epilogues, which add every term to the FP64 sums,
-    // keep those in shared memory (lane-owned, no atomics), leaving registers to the
-    // walk and the E vectors.
+    // FP32 and round the block partials: the FP32 pair phase, one sine / cosine and two
+    // FMAs per (ray, channel), no conversions.  Their int64 sums stay in registers
+    // (measured on B200 with FP64 sums against shared memory: aircraft 14,198 vs 14,035
+    // samples/s, HH + VV aircraft 11,689 vs 11,268).  The FP64 polarised lane-owned
+    // epilogue, which rounds every term, keeps its sums in shared memory (lane-owned, no
+    // atomics), leaving registers to the walk and the E vectors.
     constexpr bool PART = TRANSPOSED && PREC == SBR_PREC_MIXED;
     constexpr bool SACC = TRANSPOSED && POL && !PART;
-    __shared__ double2 s_acc[SACC ? (kCtaThreads / 32) * NACC * 32 : 1];
-    double2* const my_acc = s_acc + (SACC ? (threadIdx.x >> 5) * NACC * 32 + lane : 0);
+    __shared__ longlong2 s_acc[SACC ? (kCtaThreads / 32) * NACC * 32 : 1];
+    longlong2* const my_acc = s_acc + (SACC ? (threadIdx.x >> 5) * NACC * 32 + lane : 0);
     const int rep = warp_global % P.n_rep;
     uint32_t err = 0;
     int iter = 0;
@@ -226,12 +226,12 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
         const int i_end = G.i0 + G.ni, j_end = G.j0 + G.nj;
         const int KC = K * NPOL;  // channels of this item
 
-        double accRe[SACC ? 1 : NACC], accIm[SACC ? 1 : NACC];
+        long long accRe[SACC ? 1 : NACC], accIm[SACC ? 1 : NACC];
         float pRe[PART ? NACC : 1], pIm[PART ? NACC : 1];
 #pragma unroll
         for (int c = 0; c < NACC; ++c) {
-            if constexpr (SACC) my_acc[c * 32] = make_double2(0.0, 0.0);
-            else { accRe[c] = 0.0; accIm[c] = 0.0; }
+            if constexpr (SACC) my_acc[c * 32] = make_longlong2(0, 0);
+            else { accRe[c] = 0; accIm[c] = 0; }
             if constexpr (PART) { pRe[c] = 0.0f; pIm[c] = 0.0f; }
         }
         unsigned cRays = 0, cHit = 0, cBounce = 0, cQuery = 0;
@@ -344,9 +344,13 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
 #pragma unroll
                     for (int ch = 0; ch < NACC; ++ch) {
                         if (ch < KC) {
-                            if constexpr (POL)
-                                po_term_pol(PREC, F[ch >> 1], out.Lp, out.Lh, out.Ll, out.pa[ch & 1], accRe[ch], accIm[ch]);
-                            else po_term(PREC, F[ch], out, accRe[ch], accIm[ch]);
+                            const FreqConst& Fc = F[POL ? ch >> 1 : ch];
+                            double re = 0.0, im = 0.0;
+                            if constexpr (POL) po_term_pol(PREC, Fc, out.Lp, out.Lh, out.Ll, out.pa[ch & 1], re, im);
+                            else po_term(PREC, Fc, out, re, im);
+                            const double u = units_per<PREC>(Fc, G);
+                            accRe[ch] += __double2ll_rn(re * u);
+                            accIm[ch] += __double2ll_rn(im * u);
                         }
                     }
                 }
@@ -377,7 +381,7 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
                     }
                 }
             } else {
-                // the same broadcast with the FP32 / FP64 terms summed in FP64
+                // the same broadcast with every FP32 / FP64 term rounded
                 unsigned m = __ballot_sync(FULL, done && out.amp != 0.0f);
                 while (m) {
                     const int src = __ffs(m) - 1;
@@ -400,12 +404,18 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
                     for (int c = 0; c < NACC; ++c) {
                         const int ch = c * 32 + lane;
                         if (ch < KC) {
-                            if constexpr (SACC)
-                                po_term_pol(PREC, F[ch >> 1], q.Lp, 0.0f, 0.0f, q.pa[ch & 1], my_acc[c * 32].x,
-                                            my_acc[c * 32].y);
-                            else if constexpr (POL)
-                                po_term_pol(PREC, F[ch >> 1], q.Lp, 0.0f, 0.0f, q.pa[ch & 1], accRe[c], accIm[c]);
-                            else po_term(PREC, F[ch], q, accRe[c], accIm[c]);
+                            const FreqConst& Fc = F[POL ? ch >> 1 : ch];
+                            double re = 0.0, im = 0.0;
+                            if constexpr (POL) po_term_pol(PREC, Fc, q.Lp, 0.0f, 0.0f, q.pa[ch & 1], re, im);
+                            else po_term(PREC, Fc, q, re, im);
+                            const double u = units_per<PREC>(Fc, G);
+                            if constexpr (SACC) {
+                                my_acc[c * 32].x += __double2ll_rn(re * u);
+                                my_acc[c * 32].y += __double2ll_rn(im * u);
+                            } else {
+                                accRe[c] += __double2ll_rn(re * u);
+                                accIm[c] += __double2ll_rn(im * u);
+                            }
                         }
                     }
                 }
@@ -418,12 +428,11 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
                 if constexpr (PART) {
 #pragma unroll
                     for (int c = 0; c < NACC; ++c) {
-                        if constexpr (SACC) {
-                            my_acc[c * 32].x += double(pRe[c]);
-                            my_acc[c * 32].y += double(pIm[c]);
-                        } else {
-                            accRe[c] += double(pRe[c]);
-                            accIm[c] += double(pIm[c]);
+                        const int ch = c * 32 + lane;
+                        if (ch < KC) {
+                            const double u = units_per<PREC>(F[POL ? ch >> 1 : ch], G);
+                            accRe[c] += __double2ll_rn(double(pRe[c]) * u);
+                            accIm[c] += __double2ll_rn(double(pIm[c]) * u);
                         }
                         pRe[c] = 0.0f;
                         pIm[c] = 0.0f;
@@ -433,24 +442,23 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
             }
         }
 
-        // ---- fold the item: lanes -> warp in a fixed order, then fixed point.
+        // ---- add the item's integer sums.
         // Channel ch of sample (sbase + k) lives at accumulator (sbase * NPOL + ch).
         const long long cbase = (G.sample_base + kb) * NPOL;
         if constexpr (!TRANSPOSED) {
 #pragma unroll
             for (int ch = 0; ch < NACC; ++ch) {
                 if (ch < KC) {
-                    double a = accRe[ch], b = accIm[ch];
+                    long long a = accRe[ch], b = accIm[ch];
 #pragma unroll
                     for (int off = 16; off > 0; off >>= 1) {
                         a += __shfl_xor_sync(FULL, a, off);
                         b += __shfl_xor_sync(FULL, b, off);
                     }
                     if (lane == ch) {
-                        const double invQ = fold_factor<PREC>(F[POL ? ch >> 1 : ch]);
                         unsigned long long* A = P.acc + 2 * ((cbase + ch) * P.n_rep + rep);
-                        add_fixed(A, a, invQ);
-                        add_fixed(A + 1, b, invQ);
+                        add_fixed(A, a);
+                        add_fixed(A + 1, b);
                     }
                 }
             }
@@ -459,14 +467,13 @@ __global__ void __launch_bounds__(kCtaThreads, min_ctas_per_sm<EPI>()) k_trace(c
             for (int c = 0; c < NACC; ++c) {
                 const int ch = c * 32 + lane;
                 if (ch < KC) {
-                    const double invQ = fold_factor<PREC>(F[POL ? ch >> 1 : ch]);
                     unsigned long long* A = P.acc + 2 * ((cbase + ch) * P.n_rep + rep);
                     if constexpr (SACC) {
-                        add_fixed(A, my_acc[c * 32].x, invQ);
-                        add_fixed(A + 1, my_acc[c * 32].y, invQ);
+                        add_fixed(A, my_acc[c * 32].x);
+                        add_fixed(A + 1, my_acc[c * 32].y);
                     } else {
-                        add_fixed(A, accRe[c], invQ);
-                        add_fixed(A + 1, accIm[c], invQ);
+                        add_fixed(A, accRe[c]);
+                        add_fixed(A + 1, accIm[c]);
                     }
                 }
             }
