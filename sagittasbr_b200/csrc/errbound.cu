@@ -34,10 +34,17 @@
 // exceeded with probability below 4 exp(-lambda^2 / 2) (lambda = 6: 6e-8).  Per
 // sample
 //   E_k = |Delta_k| + |S_k| (2 k c1 + eps) + lambda scale_k (2 k sqrt(Q1) + sqrt(Q0))
-//         + (items + 1) quantum_k,
-//         + lambda scale_k u sqrt(Q2),
-// Q1 = sum (amp (dL - dLs))^2, Q0 = sum damp^2 over the rounding-only rays; the
-// fixed-point term covers the fixed-point fold of the sweep.  The last term covers
+//         + fixed_k + lambda scale_k u sqrt(Q2),
+// Q1 = sum (amp (dL - dLs))^2, Q0 = sum damp^2 over the rounding-only rays.  fixed_k
+// covers the sweep's fixed-point sums: each of the N rays (or each group of them) is
+// rounded once, within half a unit of the sample in the real and in the imaginary part,
+// whatever items and launches it ran in.  Roundings of different terms count as
+// independent: lambda sqrt(N / 2) units, and one for the final conversion.  Those of
+// equal terms add coherently like eps, by at most sqrt(1/2) N units in all, which is
+// 2^-31.5 of their sum for the largest grid (2^31 rays of 2^-62) and lies within what eps
+// has over its parts.  fixed_k is the larger of that and 2^-60 of the field's bound per
+// run of blocks, which covers it from about 1,150 rays on and is what a statement of the
+// same run always held.  The last term covers
 // the FP32 partial sums of the lane-owned epilogue: each term of a 4x8 ray block is
 // added to its channel's FP32 partial by one FMA, rounded within u |partial|, and
 // every partial is within A_b = sum |amp| of the block, so Q2 = sum over blocks of
@@ -532,10 +539,11 @@ extern "C" sbr_status sbr_error_bound(sbr_scene* s, const sbr_job* jobs, size_t 
         for (int64_t g = 0; g < p->n_segs; ++g) {
             const Segment& G = p->segs[(size_t)g];
             const JobConst& J = p->jobs[(size_t)G.job];
-            // folds of the sweep, in runs of blocks; a run's items (cut_items) round it several
-            // times, independently, by at most half a unit each
+            // the fixed-point term in units of the job
             const int run = o.blocks_per_item > 0 ? G.blocks_per_item : auto_run(G.blocks);
-            const int64_t items = (G.blocks + run - 1) / run;
+            const int64_t runs = (G.blocks + run - 1) / run;
+            const double rays = double((int64_t)G.ni * G.nj);
+            const double fixed = std::max(4.0 * double(runs + 1), (kLambda * std::sqrt(0.5 * rays) + 1.0) / double(G.finer));
             for (int k = 0; k < J.n_freqs; ++k) {
                 const FreqConst& F = p->freqs[(size_t)(J.freq_base + k)];
                 const int64_t smp = G.sample_base + k;
@@ -544,7 +552,7 @@ extern "C" sbr_status sbr_error_bound(sbr_scene* s, const sbr_job* jobs, size_t 
                 const double shared = a * ((A[0] > 0.0 ? 2.0 * F.k * A[1] / A[0] : 0.0) + kPhaseEps);
                 const double E = std::hypot(dfield[2 * smp], dfield[2 * smp + 1]) + shared +
                                  kLambda * F.scale * (2.0 * F.k * std::sqrt(A[3]) + std::sqrt(A[4])) +
-                                 4.0 * double(items + 1) * F.quantum + kLambda * F.scale * double(kU) * std::sqrt(A[2]);
+                                 fixed * F.quantum + kLambda * F.scale * double(kU) * std::sqrt(A[2]);
                 if (err_field) err_field[smp] = E;
                 if (err_db) {
                     const double db = 10.0 * std::log10(std::max(4.0 * M_PI * a * a, 1e-10));
