@@ -87,7 +87,7 @@ __device__ __forceinline__ void adjoint_ray(const AdjointParams& P, const Segmen
         r.count = 0;
         if (valid) start_f<PREC>(r, G, J, i, j);
         while (__any_sync(FULL, walking))
-            if (walking) walking = !step_f<PREC, true, false, false, false, true>(r, e, P.S, J.max_bounces, err, &rec, nullptr, nullptr);
+            if (walking) walking = !step_f<PREC, true, false, false, true>(r, e, P.S, J.max_bounces, err, &rec, nullptr, nullptr);
         n = valid ? r.count : 0;
     }
     if (n == 0) return;

@@ -133,12 +133,10 @@ constexpr unsigned long long kZWalk = 0xfffffffe00000000ull;
 // One closest-hit query, then reflect and nudge; true when the ray is finished.
 // The first query is read from the first-hit buffer when there is one (a tile no
 // triangle reaches has no entries there).
-// SPEC: the speculative closest-hit walk, entered by all lanes of `mask` together.
 // F2: slab planes two-wide (see Walker<false>).
-template <int PREC, bool REC, bool POL, bool W8 = false, bool SPEC = false, bool F2 = !REC>
+template <int PREC, bool REC, bool POL, bool W8 = false, bool F2 = !REC>
 __device__ __forceinline__ bool step_f(RayF& r, PolF& e, const SceneView& S, int maxB, uint32_t& err,
-                                       sbr_ray_record* rec, const unsigned long long* zbuf, const uint32_t* tile_cnt,
-                                       unsigned mask = 0u) {
+                                       sbr_ray_record* rec, const unsigned long long* zbuf, const uint32_t* tile_cnt) {
     if (PREC == SBR_PREC_MIXED && r.zidx < 0) return true;
     float tB = 1e20f;
     int slot;
@@ -148,9 +146,6 @@ __device__ __forceinline__ bool step_f(RayF& r, PolF& e, const SceneView& S, int
     if (key != kZWalk) {
         tB = __uint_as_float((unsigned)(key >> 32));
         slot = (int)(unsigned)key;
-    } else if constexpr (SPEC) {
-        static_assert(PREC == SBR_PREC_MIXED && !REC && !POL && !W8, "the speculative walk is the mixed scalar sweep's");
-        slot = closest_speculative(S, r.o, r.d, 1.0e-3f, tB, err, mask);
     } else if constexpr (W8) {
         static_assert(PREC == SBR_PREC_MIXED && !REC && !POL, "the 8-wide walk is the mixed scalar sweep's");
         slot = Walker8::closest(S, r.o, r.d, 1.0e-3f, tB, err);
