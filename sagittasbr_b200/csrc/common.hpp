@@ -102,7 +102,7 @@ struct SceneView {
     const int32_t* __restrict__ tri_id;
     const GNode8* __restrict__ nodes8;  // the 8-wide tree of the same leaves, or null
     const int32_t* __restrict__ tie;    // per slot: rank in the reference's walk order, or null
-    const unsigned long long* __restrict__ horizon;  // per slot: a byte per octant of directions (horizon.cu)
+    const unsigned long long* horizon;  // per slot: a byte per octant of directions (horizon.cu)
     const int32_t* __restrict__ leaf_of;  // with tris64: per slot, 4 * node + child of its leaf
     float reach;  // at least the largest coordinate of the scene's bounds
 };

@@ -58,7 +58,7 @@
 #include <cmath>
 
 #include "plan.hpp"
-#include "trace.cuh"
+#include "ray.cuh"
 
 namespace sbr {
 namespace {
@@ -152,7 +152,7 @@ __device__ __forceinline__ void add_tri(const HorizonTri& T, const GTri& X, Oct&
 }
 
 __global__ void __launch_bounds__(128) k_horizon(const GNode4* __restrict__ nodes, const GTri* __restrict__ tris,
-                                                 int64_t ntris, unsigned long long* __restrict__ out) {
+                                                 int64_t ntris, unsigned long long* out) {
     const int64_t slot = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (slot >= ntris) return;
     // the scene's bounds from the root's children
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(128) k_horizon(const GNode4* __restrict__ node
     const float flat = fmaxf(fabsf(dot(ab, T.n)), fabsf(dot(ac, T.n)));
     T.off = flat - (1.0e-4f - en);
     if (!(dot(T.n, T.n) > 0.9f) || !(4.0f * kU32 * (far + lmax) <= 4.0e-3f * alt) || !(T.off <= -2.0e-5f)) {
-        out[slot] = ~0ull;
+        store_horizon(out + slot, ~0ull);
         return;
     }
     T.lo = f3(min3f(T.a.x, b.x, c.x), min3f(T.a.y, b.y, c.y), min3f(T.a.z, b.z, c.z));
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(128) k_horizon(const GNode4* __restrict__ node
     }
     // 0.01 above the bound: the roundings of this pass and of the ray's own d.n
     unsigned long long v = (unsigned long long)__vaddus4(H.b, 0x03030303u) << 32 | __vaddus4(H.a, 0x03030303u);
-    out[slot] = over ? ~0ull : v;
+    store_horizon(out + slot, over ? ~0ull : v);
 }
 
 }  // namespace

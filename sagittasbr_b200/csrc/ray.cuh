@@ -95,6 +95,18 @@ __device__ __forceinline__ F3 primary_origin(const Segment& G, const JobConst& J
     }
 }
 
+// A triangle's horizon bytes.  k_horizon may write them while sweeps of other streams run
+// (such a sweep sees 255 or the final bytes): the loads and stores are relaxed ones at the
+// scope of the device, not read-only loads.
+__device__ __forceinline__ unsigned long long load_horizon(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void store_horizon(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" : : "l"(p), "l"(v) : "memory");
+}
+
 // Whether a ray that triangle `slot` reflected (n: its normal, d: the new direction,
 // unit) is known to meet nothing: it left the front side (cosl > 0) and rises above
 // the triangle's horizon in its octant of directions (horizon.cu).  Its next query
@@ -102,7 +114,7 @@ __device__ __forceinline__ F3 primary_origin(const Segment& G, const JobConst& J
 __device__ __forceinline__ bool leaves_scene(const SceneView& S, int slot, float cosl, float dx, float dy, float dz,
                                              float dn) {
     const unsigned o = (__float_as_uint(dx) >> 31) | (__float_as_uint(dy) >> 31) << 1 | (__float_as_uint(dz) >> 31) << 2;
-    return cosl > 0.0f && dn * kHorizonUnit > float(unsigned(__ldg(S.horizon + slot) >> (8 * o)) & 255u);
+    return cosl > 0.0f && dn * kHorizonUnit > float(unsigned(load_horizon(S.horizon + slot) >> (8 * o)) & 255u);
 }
 
 // First-hit buffer entry of ray (i, j): tile-major, the lane of the 4x8 block last.
