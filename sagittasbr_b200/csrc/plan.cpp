@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <iterator>
 
 #include "plan.hpp"
 
@@ -377,7 +378,9 @@ sbr_status plan_create(sbr_scene* const* scenes, size_t n_scenes, const int32_t*
 // Autotuner of batched plans: every candidate (blocks per work item, persistent
 // CTAs per SM) -- the automatic setting among them -- runs a sample of the plan
 // (up to 128 angles spread evenly over the jobs' angle lists) twice, the second
-// run timed on the device, and the fastest setting is written into `o`.
+// run timed on the device, and the fastest setting is written into `o`.  The candidates'
+// rays are counted towards the scenes' horizons before the first of them runs and not
+// again, so that all run on scenes in one state and none pays for the horizons.
 sbr_status autotune(sbr_scene* const* scenes, size_t n_scenes, const int32_t* job_scene, const sbr_job* jobs,
                     size_t n_jobs, sbr_run_opts& o) {
     const int64_t per_job = std::max<int64_t>(2, 128 / (int64_t)std::max<size_t>(1, n_jobs));
@@ -401,6 +404,7 @@ sbr_status autotune(sbr_scene* const* scenes, size_t n_scenes, const int32_t* jo
     if (!job_scene && o.node_width == 0 && scenes[0]->d_nodes8) widths = {4, 8};
     double best = INFINITY;
     int best_bpi = 0, best_ctas = 0, best_w = o.node_width;
+    bool counted = false;
     for (int w : widths)
     for (int c : ctas) {
         for (int b : bpis) {
@@ -413,6 +417,12 @@ sbr_status autotune(sbr_scene* const* scenes, size_t n_scenes, const int32_t* jo
             sbr_plan* pl = nullptr;
             sbr_status st = plan_create(scenes, n_scenes, job_scene, sj.data(), n_jobs, &t, &pl);
             if (st != SBR_OK) return st;
+            if (!counted) {
+                for (auto& sr : pl->scene_rays) sr.second *= 2 * (int64_t)(widths.size() * std::size(ctas) * std::size(bpis));
+                st = plan_horizons(pl);
+                counted = true;
+            }
+            pl->scene_rays.clear();
             sbr_result r{};
             for (int rep = 0; rep < 2 && st == SBR_OK; ++rep) {
                 st = sbr_plan_execute(pl);
