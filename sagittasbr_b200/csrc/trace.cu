@@ -1074,8 +1074,13 @@ sbr_status plan_launch(sbr_plan* pl, bool records, sbr_ray_record* d_records) {
             // the reference loop: one trace + PO launch per (angle, frequency), each
             // with its own queue head.  The launches do not depend on one another (their
             // accumulators are apart) and each is as long as its slowest ray: they go round
-            // the scene's side streams, between a fork from and a join to the plan's.
-            sbr_status fs = plan_fork(pl);
+            // the scene's side streams, between a fork from and a join to the plan's.  Into a
+            // caller's graph they go one after another: until the capture ends, the side
+            // streams would belong to it and refuse the scene's other plans.
+            cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+            SBR_CUDA(cudaStreamIsCapturing(st, &capturing));
+            const bool forks = capturing == cudaStreamCaptureStatusNone;
+            sbr_status fs = forks ? plan_fork(pl) : SBR_OK;
             if (fs != SBR_OK) return fs;
             for (size_t g = 0; g < pl->segs.size(); ++g) {
                 const Segment& G = pl->segs[g];
@@ -1090,12 +1095,12 @@ sbr_status plan_launch(sbr_plan* pl, bool records, sbr_ray_record* d_records) {
                     p.item_end = pl->seg_base[g + 1];
                     p.queue = pl->d_queue + 1 + G.sample_base + k;
                     const int grid = (int)std::min<long long>(pl->persistent_grid, (n + 3) / 4);
-                    sbr_status s = launch_trace(fn, grid, pl->side[launches % pl->n_side], p);
+                    sbr_status s = launch_trace(fn, grid, forks ? pl->side[launches % pl->n_side] : st, p);
                     if (s != SBR_OK) return s;
                     ++launches;
                 }
             }
-            if ((fs = plan_join(pl)) != SBR_OK) return fs;
+            if (forks && (fs = plan_join(pl)) != SBR_OK) return fs;
         }
     }
     finalize(pl->n_samples * npol, kAccReplicas, pl->d_quantum, pl->d_acc, pl->d_field, (long long)pl->n_segs * 4,
