@@ -467,12 +467,16 @@ extern "C" sbr_status sbr_error_bound(sbr_scene* s, const sbr_job* jobs, size_t 
     Parts parts;
     const size_t acc_at = parts.add(acc.size() * sizeof(double)), df_at = parts.add(dfield.size() * sizeof(double)),
                  queue_at = parts.add(2 * sizeof(unsigned long long)), zero_b = parts.add(0);
-    // a launch takes as many items as the list of flagged rays has room for
+    // a launch takes as many items as the list of flagged rays has room for, which is
+    // halved until the device has the memory
     const long long run = std::max<int64_t>(1, p->n_items > 0 ? *std::max_element(run_blocks.begin(), run_blocks.end()) : 1);
-    const long long per_launch = std::max<long long>(1, std::min<long long>(p->n_items, kFlaggedMax / (32 * run)));
-    const size_t flag_at = parts.add((size_t)(per_launch * run * 32) * sizeof(Flagged));
+    long long per_launch = std::max<long long>(1, std::min<long long>(p->n_items, kFlaggedMax / (32 * run)));
+    const size_t flag_at = parts.add(0);
     char* block = nullptr;
-    cudaError_t e = pool_alloc(p->device, &block, parts.size());
+    cudaError_t e;
+    while ((e = pool_alloc(p->device, &block, flag_at + (size_t)(per_launch * run * 32) * sizeof(Flagged))) ==
+               cudaErrorMemoryAllocation && per_launch > 1)
+        per_launch = (per_launch + 1) / 2;
     if (e != cudaSuccess) st = fail(SBR_ERR_OOM, "error-bound accumulators");
     if (st == SBR_OK) {
         d_acc = reinterpret_cast<double*>(block + acc_at);

@@ -1,4 +1,4 @@
-"""The stated error: its fixed-point term."""
+"""The stated error: on little memory, and its fixed-point term."""
 import numpy as np
 import pytest
 
@@ -12,6 +12,32 @@ pytestmark = pytest.mark.gpu
 def _cuda():
     import torch
     assert torch.cuda.is_available(), "GPU tests need a CUDA device"
+
+
+def test_the_list_of_flagged_rays_shrinks_to_the_memory_there_is():
+    """17 M rays list up to 400 MB at once; with less free, they go in several launches."""
+    import torch
+    v, t = M.ellipsoid_sh(n_theta=40, n_phi=80)
+    G = 2.0 * M.bounding_radius(v)
+    small = sbr.JobSpec([80.0], [10.0], [5e9], 100, 100, G, 4)
+    job = sbr.JobSpec(np.full(24, 80.0), np.linspace(0.0, 90.0, 24), [5e9], 2000, 2000, G, 4)
+    with sbr.Scene(v, t, want_fp64=True) as s:
+        sbr.error_bound(s, small, sbr.run(s, small))  # code and stacks of the kernels are on the device
+        r = sbr.run(s, job, first_hit=sbr.FIRST_HIT_TRAVERSE)
+        assert int(r.stats[:, 0].sum()) > 17_000_000
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        rest = torch.empty(max(0, free - (200 << 20)), dtype=torch.uint8, device="cuda")
+        try:
+            little = sbr.error_bound(s, job, r)
+        finally:
+            del rest
+            torch.cuda.empty_cache()
+        plenty = sbr.error_bound(s, job, r)
+    # sums of the same terms in another order
+    for a, b in zip(little, plenty):
+        np.testing.assert_allclose(a, b, rtol=1e-9)
 
 
 @pytest.mark.parametrize("nx, n", [(2, 1), (4, 3), (12, 1), (30, 2), (230, 3), (300, 90), (1500, 2)])
