@@ -430,7 +430,10 @@ sbr_status sbr_scene_create(const float* xyz, size_t nverts, const uint32_t* tri
     if (rb) s->d_tie = reinterpret_cast<int32_t*>(b + tie_at);
     s->d_err = reinterpret_cast<uint32_t*>(b + err_at);
     // cancel flag: a device word (the kernels poll it from L2); the host sets it on a side
-    // stream, which runs while the sweep kernel is resident
+    // stream while the sweep kernel holds every SM.  The driver writes a single word without
+    // one (measured on B200, driver 580: a sweep with the whole register file in use ends at
+    // its warps' next items).  The 8 pinned bytes that a copy would need cost 1 to 3 ms a
+    // scene to allocate and 0.5 ms to free
     s->d_cancel = reinterpret_cast<int32_t*>(b + cancel_at);
     if (collapse_on_gpu) {
         e = cudaMemcpyAsync(s->d_tri_id, gt.order, ib, cudaMemcpyDeviceToDevice, s->stream);

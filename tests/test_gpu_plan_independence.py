@@ -48,16 +48,33 @@ def test_an_angle_alone_and_among_others(nx, ny, n, prec, nf):
             np.testing.assert_array_equal(one.stats[0], whole.stats[k])
 
 
+@pytest.mark.parametrize("nf", [1, 40])
+@pytest.mark.parametrize("first_hit", [sbr.FIRST_HIT_TRAVERSE, sbr.FIRST_HIT_RASTER])
+def test_every_cut_of_large_angles(nf, first_hit):
+    """Angles of 276,000 blocks, 58 for each resident warp: 1, 10 and 36 of them are cut into
+    items of 2, 4 and 8 blocks, ragged at both edges.  With many channels the items share runs
+    of 8 blocks."""
+    v, t = M.icosphere(4, 1.0)
+    th, ph = np.linspace(60.0, 100.0, 36), np.linspace(0.0, 200.0, 36)
+    fr = np.linspace(1e9, 3e9, nf)
+    with sbr.Scene(v, t) as s:
+        runs = [sbr.run(s, sbr.JobSpec(th[:n], ph[:n], fr, 3001, 2941, 2.01, 3), first_hit=first_hit)
+                for n in (1, 10, 36)]
+    for few, many in zip(runs, runs[1:]):
+        np.testing.assert_array_equal(many.field[:few.field.size], few.field)
+        np.testing.assert_array_equal(many.stats[:few.stats.shape[0]], few.stats)
+
+
 @pytest.mark.parametrize("nf", [1, 3])
-def test_largest_items_and_polarised(nf):
-    """Angles of half a million blocks, and (HH, VV) sweeps."""
+def test_polarised(nf):
     v, t = M.icosphere(4, 1.0)
     th, ph = np.linspace(60.0, 100.0, 4), np.linspace(0.0, 200.0, 4)
-    with sbr.Scene(v, t) as s:
-        for nx, pol in ((4200, sbr.POL_SCALAR), (700, sbr.POL_HHVV), (130, sbr.POL_HHVV)):
-            fr = np.linspace(1e9, 3e9, nf)
-            whole = sbr.run(s, sbr.JobSpec(th, ph, fr, nx, nx - 3, 2.1, 3), polarization=pol)
-            one = sbr.run(s, sbr.JobSpec(th[2:3], ph[2:3], fr, nx, nx - 3, 2.1, 3), polarization=pol)
+    fr = np.linspace(1e9, 3e9, nf)
+    with sbr.Scene(v, t, want_fp64=True) as s:
+        for nx, prec in ((700, sbr.PREC_MIXED), (130, sbr.PREC_MIXED), (130, sbr.PREC_FP64)):
+            whole = sbr.run(s, sbr.JobSpec(th, ph, fr, nx, nx - 3, 2.1, 3), precision=prec, polarization=sbr.POL_HHVV)
+            one = sbr.run(s, sbr.JobSpec(th[2:3], ph[2:3], fr, nx, nx - 3, 2.1, 3), precision=prec,
+                          polarization=sbr.POL_HHVV)
             np.testing.assert_array_equal(one.field, whole.field[2 * nf:3 * nf])
 
 
