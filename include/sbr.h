@@ -132,18 +132,20 @@ typedef struct sbr_job {
                                  frequencies of a job come from one trace */
 #define SBR_MODE_PER_ANGLE 1  /* the reference's loop: one trace + PO launch per (angle, frequency) */
 
-#define SBR_PREC_MIXED 0      /* FP32 traversal, FP64 path length, FP32-pair phase reduction, FP64 field sums */
+#define SBR_PREC_MIXED 0      /* FP32 traversal, FP64 path length, FP32-pair phase reduction, fixed-point field sums */
 #define SBR_PREC_FP32 1       /* the reference FP32 build's arithmetic (launch plane at 10 G, FP32 phase) */
-#define SBR_PREC_FP64 2       /* everything in FP64 (the reference USE_DOUBLE build's arithmetic) */
+#define SBR_PREC_FP64 2       /* rays, triangle tests, paths, phases and terms in FP64 (the reference
+                                 USE_DOUBLE build's arithmetic).  The tree's boxes, which only prune, are
+                                 tested in FP32 with margins that cover the roundings, and the leaf of
+                                 every hit in FP64; the hits are those of FP64 box tests */
 
 /* How the first closest hit of each ray is found.  Primary rays of one angle are
  * parallel and start on the launcher grid, so their first hits form an
  * orthographic z-buffer: RASTER tests every triangle against the pixels its
- * projection covers (same Moller-Trumbore arithmetic) and keeps the nearest per
- * pixel; later bounces always walk the BVH.  RASTER applies to batched FP32 /
- * mixed runs (per-angle and FP64 runs always walk).  Measured on B200 it costs
- * about as much as the walk it replaces for coherent ray tubes, so the default
- * walks. */
+ * projection covers (the walk's own triangle test) and keeps the nearest per
+ * pixel; later bounces always walk the BVH.  RASTER applies to batched mixed
+ * runs over one scene (the others always walk).  It costs per triangle and angle
+ * and saves per ray, hence the automatic rule. */
 #define SBR_FIRST_HIT_AUTO 0      /* (default) the raster where a plan launches, per angle, at least
                                      8 rays per triangle of its scene; the walk otherwise */
 #define SBR_FIRST_HIT_RASTER 1    /* first hits from the tile-binned orthographic raster (batched
@@ -172,7 +174,13 @@ typedef struct sbr_run_opts {
     int32_t ctas_per_sm;      /* persistent grid size per SM; 0 -> occupancy-derived */
     int32_t first_hit;        /* SBR_FIRST_HIT_* */
     int32_t blocks_per_item;  /* 32-ray blocks (4 x 8) per work item; 0 -> automatic (batched: blocks / 1024
-                                 clamped to 1..8 per angle, per-angle mode: 1) */
+                                 clamped to 1..8 per angle, cut down to 1, 2 or 4 where the whole sweep has
+                                 few blocks per resident warp; per-angle mode: 1).  A field does not depend
+                                 on the automatic cut: every ray's term (in mixed sweeps of more than four
+                                 channels, the FP32 sum of each group of 32 rays, formed within runs of
+                                 blocks / 1024 clamped to 1..8) is rounded to a fixed-point unit of its
+                                 sample and summed as an integer.  An angle has the same bits alone, in a
+                                 shard and in any plan with the same options and largest channel count */
     int32_t autotune;         /* 1: sbr_plan_create times candidate (blocks_per_item, ctas_per_sm)
                                  settings -- and both tree widths when the scene holds an 8-wide
                                  tree -- on a sample of the plan's angles and keeps the fastest

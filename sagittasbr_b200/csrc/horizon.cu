@@ -35,9 +35,11 @@
 // triangle.  They cost 5 to 15 ns a triangle and save 2 to 130 ps a launched ray (break-even
 // at 60 rays per triangle on a smooth ellipsoid, 120 on a small sphere, 650 on a coarse
 // aircraft, 3,900 on a fine jittered one seen from the nose), and a ray costs 30 to 100 ps:
-// at 1,500 the sweep that brings them is at most a tenth longer for it, and a first look at
-// a new model, or a step that moves the vertices again, does not pay for what it cannot
-// use (at 200 a first sweep took up to 36 % longer).
+// by then a scene's sweeps have taken 45 to 150 ns a triangle, so the build is 3 to 33 % of
+// them once.  It falls on the sweep that reaches the count, however short that one is (a
+// single look at the full-size aircraft can take 21 ms longer).  A first look at a new
+// model, or a step that moves the vertices again, does not pay for what it cannot use (at
+// 200 a first sweep took up to 36 % longer).
 // The bytes change in place: a plan or graph made before reads them too, and a kernel that
 // runs meanwhile sees 255 or the final byte.
 //

@@ -343,11 +343,14 @@ struct PlanSink : sbr::TableSink {
 // Cuts a batched plan's automatic work items down to 1, 2, 4 or 8 blocks: a launch ends
 // when its slowest warps have finished the items they took last, and items of 8 blocks
 // with a few five-bounce rays among them run for most of a millisecond.  With few blocks
-// per resident warp that end weighs most, with many the items' own set-up and fold.  Measured on B200 (blocks per resident warp: ms at items of 1 /
-// 2 / 4 / 8 blocks): sphere (11) 0.457 / 0.476 / 0.521 / 0.564, plates (55) 2.40 / 2.47 /
-// 2.72 / 3.11, ellipsoid (65) 2.21 / 2.19 / 2.21 / 2.40, narrow aircraft (261) 2.97 / 2.77
-// / 3.15 / 3.30, HH + VV aircraft (578) 9.15 / 6.74 / 6.67 / 7.35, wideband aircraft (1570)
-// 34.7 / 24.9 / 22.8 / 23.7, its 61 azimuths (15,800) 199.5 ms at 4 and 197.2 at 8.  Sweeps with FP32 partial sums per group of rays (`groups`)
+// per resident warp that end weighs most, with many the items' own set-up and fold.
+// Measured on B200 (blocks per resident warp: ms at items of 1 / 2 / 4 / 8 blocks): sphere
+// (11) 0.457 / 0.476 / 0.521 / 0.564, plates (55) 2.40 / 2.47 / 2.72 / 3.11, ellipsoid (65)
+// 2.21 / 2.19 / 2.21 / 2.40, narrow aircraft (261) 2.97 / 2.77 / 3.15 / 3.30, HH + VV
+// aircraft (578) 9.15 / 6.74 / 6.67 / 7.35, wideband aircraft (1570) 34.7 / 24.9 / 22.8 /
+// 23.7, its 61 azimuths (15,800) 199.5 ms at 4 and 197.2 at 8; one look at the 133k
+// aircraft (6.6) 0.179 / 0.260 / 0.430 / 0.776.  The cut may look at the whole plan because
+// it changes no field (k_trace).  Sweeps with FP32 partial sums per group of rays (`groups`)
 // keep their runs of blocks, in which the groups form, and share them between items.
 void cut_items(sbr_plan* p, bool groups) {
     int64_t blocks = 0;

@@ -58,8 +58,12 @@ constexpr int kRegK = 4;     // per-lane accumulation up to this many channels
 //                         channels (registers sized to the plan's channel count)
 //   EPI_T32 / T64 / T128: lanes own channels lane, lane + 32, ...; each finished ray
 //                         is broadcast to the warp (up to 32 / 64 / 128 channels)
-// A channel's terms are added in the same order in all three, so the layout changes no
-// field; it sets the registers and the columns a broadcast ray is offered to.  Up to 32
+// The lane-owned layouts form the same groups in the same order, so which of them runs
+// changes no field as long as the compiler fuses a term's products alike in all three (it
+// does: equal bits in every precision, scalar and polarised).  In mixed precision a group's
+// FP32 sum makes them differ from the per-lane layouts by about 1e-7 of a field; FP32 and
+// FP64 sweeps have the same bits in all five.  The layout sets the registers and the columns
+// a broadcast ray is offered to.  Up to 32
 // channels EPI_T32 against EPI_T64, ms on B200: 8 scalar frequencies, aircraft of 537k
 // triangles 12.99 -> 12.15, trihedral 25.49 -> 23.76, ellipsoid 3.23 -> 3.08, sphere
 // 0.545 -> 0.513; 16 frequencies HHVV 13.81 -> 12.87, 27.59 -> 25.90, 3.34 -> 3.18,
@@ -993,7 +997,8 @@ sbr_status tile_raster(sbr_plan* pl, const sbr_plan::Chunk& ch, cudaStream_t st,
 // 20k-triangle sphere (145 blocks) 54 / 38 / 38 / 37, four 59 / 52 / 52 / 49, thirty (4,350)
 // 92 / 92 / 93 / 107, one at a 200k-triangle ellipsoid (555) 210 / 149 / 121 / 124, FP64
 // sphere 69 / 46 / 47 / 46, plates with six bounces 285 / 285 / 234 / 196.
-// Blocks whose terms are added in FP32 first (more than kRegK mixed channels) stay whole.
+// Blocks whose terms are added in FP32 first (more than kRegK mixed channels) stay whole; the
+// others' terms are rounded ray by ray, so sharing a block changes no field.
 static int lanes_log2(const sbr_plan* pl, int channels, long long items) {
     if (pl->prec == SBR_PREC_MIXED && channels > kRegK) return 5;
     for (const Segment& g : pl->segs)
