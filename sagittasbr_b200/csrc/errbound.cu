@@ -1,6 +1,6 @@
 // errbound.cu -- sbr_error_bound: the error, per (angle, frequency) sample, of the
-// mixed-precision sweep (FP32 traversal, FP64 path, FP32 phase pairs, FP64 sums of
-// FP32 block partials) against the FP64 sweep of the same job.  No counterpart in the reference, which has no
+// mixed-precision sweep (FP32 traversal, FP64 path, FP32 phase pairs, fixed-point sums
+// of the terms or of FP32 block partials) against the FP64 sweep of the same job.  No counterpart in the reference, which has no
 // mixed-precision mode.
 //
 // A second pass re-traces every ray of the plan with the mixed sweep's own
@@ -39,16 +39,17 @@
 // covers the sweep's fixed-point sums: each of the N rays (or each group of them) is
 // rounded once, within half a unit of the sample in the real and in the imaginary part,
 // whatever items and launches it ran in.  Roundings of different terms count as
-// independent: lambda sqrt(N / 2) units, and one for the final conversion.  Those of
-// equal terms add coherently like eps, by at most sqrt(1/2) N units in all, which is
-// 2^-31.5 of their sum for the largest grid (2^31 rays of 2^-62) and lies within what eps
-// has over its parts.  fixed_k is the larger of that and 2^-60 of the field's bound per
-// run of blocks, which covers it from about 1,150 rays on and is what a statement of the
-// same run always held.  The last term covers
+// independent: lambda sqrt(N / 2) units, and one for the final conversion.  fixed_k is
+// the larger of that and 2^-60 of the field's bound per run of blocks, which covers it
+// from about 1,150 rays on and is what a statement of the same run always held.  Equal
+// terms round equally, by at most sqrt(1/2) N units in all; that part adds coherently, as
+// the share sqrt(1/2) N units / (scale_k sum amp) of the field, and belongs to eps, which
+// has 3.4e-7 over its other parts (a sweep of 10^6 rays of full amplitude needs 2e-13; it
+// grows with max(1, R)^max_bounces).  The last term covers
 // the FP32 partial sums of the lane-owned epilogue: each term of a 4x8 ray block is
 // added to its channel's FP32 partial by one FMA, rounded within u |partial|, and
 // every partial is within A_b = sum |amp| of the block, so Q2 = sum over blocks of
-// n_b A_b^2 (n_b terms); the per-lane layouts sum in FP64 and the term only
+// n_b A_b^2 (n_b terms); the per-lane layouts round each term and the term only
 // overstates their error.  The phase pair's 2^-45 |x| turns (ray.cuh, turns_frac)
 // is added to dLs as 2^-45 L.
 #include <algorithm>
@@ -66,6 +67,7 @@ constexpr float kU = 5.9604644775390625e-08f;  // 2^-24, unit roundoff of FP32
 // 2 k L in turns (2 pi 2^-25 rad; the FP32 pair's 2^-45 |x| is carried in dLs),
 // __sincosf (below 4e-7 absolute), FP32 amplitude (2^-24).
 constexpr double kPhaseEps = 1.0e-6;
+constexpr double kPhaseParts = 6.6e-7;  // the sum of these
 
 constexpr double kPhaseExact = 0.05;  // rad: rays with more phase uncertainty are re-traced in FP64
 constexpr double kLambda = 6.0;       // probabilistic bound multiplier (failure below 6e-8)
@@ -553,7 +555,9 @@ extern "C" sbr_status sbr_error_bound(sbr_scene* s, const sbr_job* jobs, size_t 
                 const int64_t smp = G.sample_base + k;
                 const double* A = acc.data() + 8 * g;
                 const double a = std::hypot(field[2 * smp], field[2 * smp + 1]);
-                const double shared = a * ((A[0] > 0.0 ? 2.0 * F.k * A[1] / A[0] : 0.0) + kPhaseEps);
+                const double equal = std::sqrt(0.5) * rays * (F.quantum / double(G.finer)) / F.scale;  // of equal terms, times sum amp
+                const double shared = a * (A[0] > 0.0 ? 2.0 * F.k * A[1] / A[0] + std::max(kPhaseEps, kPhaseParts + equal / A[0])
+                                                      : kPhaseEps);
                 const double E = std::hypot(dfield[2 * smp], dfield[2 * smp + 1]) + shared +
                                  kLambda * F.scale * (2.0 * F.k * std::sqrt(A[3]) + std::sqrt(A[4])) +
                                  fixed * F.quantum + kLambda * F.scale * double(kU) * std::sqrt(A[2]);

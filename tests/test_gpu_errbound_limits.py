@@ -60,3 +60,26 @@ def test_the_fixed_point_term_covers_every_rays_rounding(nx, n):
     unit = 2.0 * k * 4.0 ** 2 / (4.0 * np.pi) / 2.0 ** 62 / share
     assert np.all(err >= (6.0 * np.sqrt(0.5 * rays) + 1.0) * unit * (1.0 - 1e-12))
     assert np.all(err <= 1e-12)
+
+
+@pytest.mark.parametrize("refl, bounces", [(1.0, 3), (30.0, 8), (100.0, 6)])
+def test_equal_terms_round_equally(refl, bounces):
+    """A plate seen face on: all rays have one path and one amplitude, so all terms are rounded
+    alike.  With a large max(1, R)^max_bounces the unit is coarse against them, and the sum of
+    the roundings is a share of the field."""
+    v = np.array([[-1, -1, 0], [1, -1, 0], [1, 1, 0], [-1, 1, 0]], dtype=np.float32)
+    t = np.array([[0, 1, 2], [0, 2, 3]], dtype=np.uint32)
+    G, n = 4.0, 201
+    f = np.linspace(1e9, 2e9, 4)
+    job = sbr.JobSpec([0.0], [0.0], f, n, n, G, bounces, refl)
+    with sbr.Scene(v, t) as s:
+        r = sbr.run(s, job)
+        err, _ = sbr.error_bound(s, job, r)
+    hits = int(r.stats[0, 1])
+    assert hits > 5000 and r.stats[0, 2] == hits
+    # path 10 G to the plate at z = 0, term k A / (4 pi) * 2 R (-sin, cos)(2 k L)
+    k = 2.0 * np.pi * f / 299792458.0
+    term = k * (G * G / (n * n)) / (4.0 * np.pi) * 2.0 * refl
+    phase = 2.0 * k * 10.0 * G
+    exact = hits * term * (-np.sin(phase) + 1j * np.cos(phase))
+    assert np.all(np.abs(r.field - exact) <= err)
