@@ -322,9 +322,10 @@ __device__ __forceinline__ float ray_bound(const ErrParams& P, int seg, const Se
         P.flagged[atomicAdd(P.n_flagged, 1ull)] = Flagged{seg, i, j, om.amp, om.Lh, om.Ll};
         ++nex;
     } else if (r.count > 0) {
-        sa += double(om.amp);
-        s1 += double(om.amp) * dLs;
-        const double e1 = double(om.amp) * (dL - dLs), e0 = 2.0 * double(fabsf(om.Rn)) * double(dnl + ua);
+        const double amp = double(fabsf(om.amp));  // (negative with a negative R and an odd count)
+        sa += amp;
+        s1 += amp * dLs;
+        const double e1 = amp * (dL - dLs), e0 = 2.0 * double(fabsf(om.Rn)) * double(dnl + ua);
         q1 += e1 * e1;
         s0 += e0 * e0;
     }

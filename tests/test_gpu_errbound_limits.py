@@ -62,7 +62,7 @@ def test_the_fixed_point_term_covers_every_rays_rounding(nx, n):
     assert np.all(err <= 1e-12)
 
 
-@pytest.mark.parametrize("refl, bounces", [(1.0, 3), (30.0, 8), (100.0, 6)])
+@pytest.mark.parametrize("refl, bounces", [(1.0, 3), (-1.0, 3), (30.0, 8), (-30.0, 8), (100.0, 6)])
 def test_equal_terms_round_equally(refl, bounces):
     """A plate seen face on: all rays have one path and one amplitude, so all terms are rounded
     alike.  With a large max(1, R)^max_bounces the unit is coarse against them, and the sum of
